@@ -41,13 +41,21 @@ struct StatAcc {
 template <typename R>
 struct CollisionParams {
   R omega;
-  R magic;
+  R omega2;  // TRT: relaxation of the antisymmetric part, trt_omega2(omega, magic)
   R smagorinsky;
   R force[3];
+  float relax[4];  // FP32 collisions: Relaxation::set
   // ConstRhoBGK: the statistics of the previous step, whose average density is the
   // AVERAGE_RHO parameter (1 while no step has been counted)
   const StatAcc* avgSrc;
 };
+
+// The second relaxation frequency of TRT (collision::TRT::apply); the same for every cell, so it is
+// found once where the parameters are set.
+template <typename R>
+__host__ __device__ __forceinline__ R trt_omega2(R omega, R magic) {
+  return R(1) / (magic / (R(1) / omega - R(0.5)) + R(0.5));
+}
 
 template <int DYN> struct DynTraits {
   static constexpr bool forced = (DYN == DYN_FORCED_BGK || DYN == DYN_FORCED_SMAGORINSKY);
@@ -153,64 +161,243 @@ __device__ __forceinline__ R smagorinsky_omega(const R (&f)[Q], R rho, const R (
   return R(1) / (tauMol + tauTurb);
 }
 
-// Collide one cell in place.  Returns the cell statistic {rho, |u|^2}.
-// FP32 BGK, written so that no product is ever an operand of a separate add: the sums of the
-// populations and of the momentum are plain adds, every product that meets an add does so inside
-// an explicit fused multiply-add.  The packed two-cell form (collide_bgk_x2) repeats this
-// sequence lane by lane, and since nothing here is left for the compiler to contract, the
-// two give the same bits.
-template <int Q>
-__device__ __forceinline__ void collide_bgk_f32(float (&f)[Q], float omega, float& rhoOut, float& uSqrOut) {
-  using D = Desc<Q>;
-  float rho = 0.f;
-  static_for<Q>([&](auto I) { rho = __fadd_rn(rho, f[I]); });
-  rho = __fadd_rn(rho, 1.f);
-  float j[3] = {0.f, 0.f, 0.f};
-  static_for<Q>([&](auto I) {
-    static_for<D::d>([&](auto A) {
-      constexpr int c = D::C[I][A];
-      if constexpr (c == 1) j[A] = __fadd_rn(j[A], f[I]);
-      else if constexpr (c == -1) j[A] = __fsub_rn(j[A], f[I]);
-    });
-  });
-  const float inv = 1.f / rho;
-  float u[3];
-  static_for<D::d>([&](auto A) { u[A] = __fmul_rn(j[A], inv); });
-  float uSqr = __fmul_rn(u[0], u[0]);
-  static_for<D::d - 1>([&](auto A) { uSqr = __fmaf_rn(u[A + 1], u[A + 1], uSqr); });
-  const float keep = 1.f - omega;
-  const float base = __fmaf_rn(-1.5f, uSqr, 1.f);
-  {
-    constexpr float t0 = weight<Q, float>(0);
-    f[0] = __fmaf_rn(omega, __fmaf_rn(__fmul_rn(rho, t0), base, -t0), __fmul_rn(f[0], keep));
+// ---- FP32 collisions, one cell or two at once ------------------------------------------------
+// The arithmetic of the FP32 and 16-bit forms, on a float (one cell) or a float2 (a pair of cells, on
+// the packed two-lane instructions of sm_100).  Every operation is an explicitly rounded add,
+// multiply or fused multiply-add, so nothing is left for the compiler to contract, and a lane of a
+// pair gets the bits of a single cell: CUDA's packed intrinsics round each component as __fadd_rn,
+// __fmul_rn and __fmaf_rn do.
+using F2 = float2;
+__device__ __forceinline__ float vadd(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float vsub(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ float vmul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float vfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ float vrcp(float a) { return 1.f / a; }
+__device__ __forceinline__ float vsqrt(float a) { return sqrtf(a); }
+__device__ __forceinline__ F2 vadd(F2 a, F2 b) { return __fadd2_rn(a, b); }
+// a - b with one rounding, as __fsub_rn: b * (-1) is exact, so the fused form rounds a + (-b) once
+__device__ __forceinline__ F2 vsub(F2 a, F2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
+__device__ __forceinline__ F2 vmul(F2 a, F2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ F2 vfma(F2 a, F2 b, F2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ F2 vrcp(F2 a) { return make_float2(1.f / a.x, 1.f / a.y); }
+__device__ __forceinline__ F2 vsqrt(F2 a) { return make_float2(sqrtf(a.x), sqrtf(a.y)); }
+template <typename V> __device__ __forceinline__ V vset(float a);
+template <> __device__ __forceinline__ float vset<float>(float a) { return a; }
+template <> __device__ __forceinline__ F2 vset<F2>(float a) { return make_float2(a, a); }
+
+// The weights of the moving directions, one class per number of non-zero components, in units of an
+// axis direction's weight t_1: exact powers of two.  With d = 3 omega t_1, N = omega / d.
+template <int Q> __host__ __device__ constexpr int weight_class(int i) {
+  return (Desc<Q>::C[i][0] != 0) + (Desc<Q>::C[i][1] != 0) + (Desc<Q>::C[i][2] != 0) - 1;
+}
+template <int Q> struct Weights {
+  static constexpr int classes = Q == 27 ? 3 : 2;
+  static constexpr float N = Q == 9 ? 3.f : (Q == 19 ? 6.f : 4.5f);      // 1 / (3 t_1)
+  static constexpr float rest = Q == 19 ? 6.f : 4.f;                     // t_0 / t_1
+  static constexpr float moving = Q == 9 ? 5.f : (Q == 19 ? 12.f : 9.5f);  // (1 - t_0) / t_1
+  static __host__ __device__ constexpr float ratio(int k) {
+    return k == 0 ? 1.f : (k == 1 ? (Q == 19 ? 0.5f : 0.25f) : 0.0625f);
   }
+};
+
+// Coefficients of the FP32 relaxation that conserve what the collision conserves to the last bit the
+// format allows: a population keeps a of itself and takes b of its opposite (BGK: b = 0), and the
+// equilibrium's even and odd parts enter with d_even, d_odd = 3 omega t_1, taken from the rounded a
+// and b, so that a + b + N d_even and a - b + N d_odd are 1.  Rounding omega t_i direction by
+// direction instead leaves a factor 1 + 3e-8 on the momentum of every step, which is most of the
+// FP32 form's error after some hundred steps.  Against FP64 after 20 steps of a 256^3 Taylor-Green
+// flow the largest relative error of a population column fell from 8.6e-5 to 3.5e-6 (with delta in
+// place of rho - 1 below), after 100 steps of a 64^3 cavity from 8.4e-6 to 2.4e-6.
+struct Relaxation {
+  static void set(int q, float omegaF, float magic, bool trt, float (&r)[4]) {
+    const double omega = omegaF, omega2 = trt ? trt_omega2(omega, double(magic)) : omega;
+    const double n = q == 9 ? 3.0 : (q == 19 ? 6.0 : 4.5);
+    r[0] = float(1.0 - 0.5 * (omega + omega2));
+    r[1] = float(0.5 * (omega2 - omega));
+    r[2] = float((1.0 - (double(r[0]) + double(r[1]))) / n);
+    r[3] = float((1.0 - (double(r[0]) - double(r[1]))) / n);
+  }
+};
+
+// BGK, TRT, Smagorinsky and the Guo-forced forms.  Opposite directions i, j share q = (c_i . J)^2
+// with J = rho u (the momentum, plus rho F / 2 where forced) and differ in the sign of what is odd in
+// c_i.  With delta = rho - 1 (the sum of the stored f - w) and K = delta - 1.5 J^2 / rho the
+// equilibrium, less w, is t (K + 4.5 q / rho +- 3 c_i . J); its constant part cancels against the
+// stored w and is never formed.  A pair of BGK costs
+//   S = omega t (K + 4.5 q / rho),  f_i' = (1 - omega) f_i + S + 3 omega t c_i . J,  f_j' likewise with -,
+// six or seven operations on coefficients that the directions of one weight share.  TRT relaxes the
+// even part with omega and the odd part with omega2: f_i' = a f_i + b f_j + S + 3 omega2 t c_i . J with
+// a = 1 - (omega + omega2) / 2, b = (omega2 - omega) / 2.  Guo's force t rho (1 - omega / 2)
+// (3 (c - u) . F + 9 (c . u) (c . F)) adds to the even part -3 u . F (shared by a weight) and
+// 9 (1 - omega / 2) t (c . F) (c . J), to the odd part 3 rho (1 - omega / 2) t c . F.
+// The 16-bit and D3Q27 forms are bounded by instruction issue (the operation order of the
+// reference's templates took 418 instructions a warp for 32 cells of D3Q19 BGK, two and three times
+// that for TRT and the forced Smagorinsky form).  At 192^3, default launch shape, FP16 D3Q27:
+// TRT 32.2k -> 39.4k MLUPS, forced Smagorinsky 25.8k -> 35.8k; with two cells a thread, which all
+// FP32 arithmetic may now pack, FP16 D3Q19 forced Smagorinsky 35.2k -> 55.8k, and the FP32
+// form of 256^3 D3Q19 BGK 37.4k -> 40.4k (0.94 of the 6542 GB/s measured on this pool).
+template <int Q, int DYN, typename V>
+__device__ __forceinline__ void collide_f32(V (&f)[Q], const CollisionParams<float>& p, V& rhoOut, V& uSqrOut) {
+  using D = Desc<Q>;
+  using T = DynTraits<DYN>;
+  using WT = Weights<Q>;
+  constexpr int NC = WT::classes;
+  V delta = f[0];
+  V j[3] = {vset<V>(0.f), vset<V>(0.f), vset<V>(0.f)};
+  V pi[6] = {vset<V>(0.f), vset<V>(0.f), vset<V>(0.f), vset<V>(0.f), vset<V>(0.f), vset<V>(0.f)};
   static_for<Q / 2>([&](auto K) {
-    constexpr int i = K + 1;
-    constexpr int jj = D::OPP[i];
-    constexpr float t = weight<Q, float>(i);
-    float cj = 0.f;  // c_i . j over the non-zero components in axis order
+    constexpr int i = K + 1, jo = D::OPP[i];
+    const V s = vadd(f[i], f[jo]), d = vsub(f[i], f[jo]);
+    delta = vadd(delta, s);
     static_for<D::d>([&](auto A) {
       constexpr int c = D::C[i][A];
-      if constexpr (c == 1) cj = __fadd_rn(cj, j[A]);
-      else if constexpr (c == -1) cj = __fsub_rn(cj, j[A]);
+      if constexpr (c == 1) j[A] = vadd(j[A], d);
+      else if constexpr (c == -1) j[A] = vsub(j[A], d);
+      if constexpr (T::smagorinsky) {
+        static_for<D::d>([&](auto B) {
+          if constexpr (B >= A) {
+            constexpr int cc = D::C[i][A] * D::C[i][B];
+            constexpr int ip = A * D::d - (A * (A - 1)) / 2 + (B - A);
+            if constexpr (cc == 1) pi[ip] = vadd(pi[ip], s);
+            else if constexpr (cc == -1) pi[ip] = vsub(pi[ip], s);
+          }
+        });
+      }
     });
-    const float cu = __fmul_rn(cj, inv);
-    const float sym = __fmaf_rn(__fmul_rn(rho, t), __fmaf_rn(__fmul_rn(4.5f, cu), cu, base), -t);
-    const float r3t = __fmul_rn(rho, 3 * t);
-    const float plus = __fmaf_rn(r3t, cu, sym), minus = __fmaf_rn(-r3t, cu, sym);
-    f[i] = __fmaf_rn(omega, plus, __fmul_rn(f[i], keep));
-    f[jj] = __fmaf_rn(omega, minus, __fmul_rn(f[jj], keep));
+  });
+  const V rho = vadd(delta, vset<V>(1.f));
+  const V inv = vrcp(rho);
+  V a = vset<V>(p.relax[0]), de = vset<V>(p.relax[2]);
+  if constexpr (T::smagorinsky) {
+    // Pi^neq with the unforced momentum j; n2 = sum of its squared components
+    V n2 = vset<V>(0.f);
+    const V third = vmul(delta, vset<V>(-1.f / 3.f));
+    static_for<D::d>([&](auto A) {
+      const V ja = vmul(j[A], inv);
+      static_for<D::d>([&](auto B) {
+        if constexpr (B >= A) {
+          constexpr int ip = A * D::d - (A * (A - 1)) / 2 + (B - A);
+          V s = vfma(vmul(ja, vset<V>(-1.f)), j[B], pi[ip]);
+          if constexpr (A == B) s = vadd(s, third);
+          if constexpr (T::forced) {
+            if constexpr (A == B) {
+              s = vfma(vset<V>(p.force[A]), j[A], s);
+            } else {
+              s = vfma(vset<V>(0.5f * p.force[A]), j[B], s);
+              s = vfma(vset<V>(0.5f * p.force[B]), j[A], s);
+            }
+          }
+          n2 = vfma(A == B ? s : vmul(s, vset<V>(2.f)), s, n2);
+        }
+      });
+    });
+    const float tau = 1.f / p.omega;
+    const float pre = p.smagorinsky * p.smagorinsky * 18.f * 1.4142135623730951f;
+    const V root = vsqrt(vfma(vmul(vset<V>(pre), inv), vsqrt(n2), vset<V>(tau * tau)));
+    // omega = 2 / (tau + root), and the coefficients of Relaxation::set for it
+    de = vmul(vrcp(vadd(root, vset<V>(tau))), vset<V>(2.f / WT::N));
+    a = vfma(vset<V>(-WT::N), de, vset<V>(1.f));
+  }
+  if constexpr (T::forced)
+    static_for<D::d>([&](auto A) { j[A] = vfma(vset<V>(0.5f * p.force[A]), rho, j[A]); });
+  V jj = vmul(j[0], j[0]);
+  static_for<D::d - 1>([&](auto A) { jj = vfma(j[A + 1], j[A + 1], jj); });
+  const V ju = vmul(jj, inv);  // rho u^2
+  const V k0 = vfma(vset<V>(-1.5f), ju, delta);
+  const V e1 = vmul(de, vset<V>(1.f / 3.f));  // omega t_1
+  V even = vmul(e1, k0);
+  V rest = vmul(vfma(vset<V>(-WT::moving), e1, vmul(de, vset<V>(WT::N))), k0);
+  const V quad = vmul(vmul(de, vset<V>(1.5f)), inv);  // 4.5 omega t_1 / rho
+  V g, h;  // forced: 9 (1 - omega / 2) t_1 and 3 rho (1 - omega / 2) t_1
+  if constexpr (T::forced) {
+    const V half = vfma(a, vset<V>(0.5f), vset<V>(0.5f));  // 1 - omega / 2
+    g = vmul(half, vset<V>(3.f / WT::N));
+    h = vmul(vmul(half, vset<V>(1.f / WT::N)), rho);
+    V jf = vmul(j[0], vset<V>(p.force[0]));
+    static_for<D::d - 1>([&](auto A) { jf = vfma(j[A + 1], vset<V>(p.force[A + 1]), jf); });
+    const V hu = vmul(vmul(h, inv), jf);
+    even = vsub(even, hu);
+    rest = vfma(vset<V>(-WT::rest), hu, rest);
+  }
+  V ce[NC], cq[NC], cd[NC], cg[NC], ch[NC];
+  const V dd = T::trt ? vset<V>(p.relax[3]) : de;
+  static_for<NC>([&](auto C) {
+    const V r = vset<V>(WT::ratio(C));
+    ce[C] = C == 0 ? even : vmul(even, r);
+    cq[C] = C == 0 ? quad : vmul(quad, r);
+    cd[C] = C == 0 ? dd : vmul(dd, r);
+    if constexpr (T::forced) {
+      cg[C] = C == 0 ? g : vmul(g, r);
+      ch[C] = C == 0 ? h : vmul(h, r);
+    }
+  });
+  f[0] = vfma(T::trt ? vset<V>(p.relax[0] + p.relax[1]) : a, f[0], rest);
+  const V b = vset<V>(p.relax[1]);
+  static_for<Q / 2>([&](auto K) {
+    constexpr int i = K + 1, jo = D::OPP[i], C = weight_class<Q>(i);
+    // c_j . J of the opposite direction, whose first non-zero component is positive
+    V cj = vset<V>(0.f);
+    float cf = 0.f;
+    bool first = true;
+    static_for<D::d>([&](auto A) {
+      constexpr int c = D::C[jo][A];
+      if constexpr (c != 0) {
+        if (first) cj = c == 1 ? j[A] : vsub(vset<V>(0.f), j[A]);
+        else cj = c == 1 ? vadd(cj, j[A]) : vsub(cj, j[A]);
+        first = false;
+        if constexpr (T::forced) cf = c == 1 ? cf + p.force[A] : cf - p.force[A];
+      }
+    });
+    V even_i, plus, minus;
+    if constexpr (T::forced) {
+      const V vcf = vset<V>(cf);
+      even_i = vfma(vfma(cq[C], cj, vmul(cg[C], vcf)), cj, ce[C]);
+      const V odd = vfma(cd[C], cj, vmul(ch[C], vcf));
+      plus = vadd(even_i, odd);
+      minus = vsub(even_i, odd);
+    } else {
+      even_i = vfma(cq[C], vmul(cj, cj), ce[C]);
+      plus = vfma(cd[C], cj, even_i);
+      minus = vfma(vmul(cd[C], vset<V>(-1.f)), cj, even_i);
+    }
+    const V fi = f[i], fj = f[jo];
+    if constexpr (T::trt) {
+      f[jo] = vfma(a, fj, vfma(b, fi, plus));
+      f[i] = vfma(a, fi, vfma(b, fj, minus));
+    } else {
+      f[jo] = vfma(a, fj, plus);
+      f[i] = vfma(a, fi, minus);
+    }
   });
   rhoOut = rho;
-  uSqrOut = uSqr;
+  uSqrOut = vmul(ju, inv);
 }
 
+// Two cells (f[k][i], k = 0, 1) of any FP32 collision but ConstRhoBGK, in place.
+template <int Q, int DYN>
+__device__ __forceinline__ void collide_x2(float (&f)[2][Q], const CollisionParams<float>& p, float (&rhoOut)[2],
+                                           float (&usqOut)[2]) {
+  F2 g[Q];
+  static_for<Q>([&](auto I) { g[I] = make_float2(f[0][I], f[1][I]); });
+  F2 rho, usq;
+  collide_f32<Q, DYN>(g, p, rho, usq);
+  static_for<Q>([&](auto I) {
+    f[0][I] = g[I].x;
+    f[1][I] = g[I].y;
+  });
+  rhoOut[0] = rho.x;
+  rhoOut[1] = rho.y;
+  usqOut[0] = usq.x;
+  usqOut[1] = usq.y;
+}
+
+// Collide one cell in place.  Returns the cell statistic {rho, |u|^2}.
 template <int Q, typename R, int DYN>
 __device__ __forceinline__ void collide(R (&f)[Q], const CollisionParams<R>& p, R& rhoOut, R& uSqrOut) {
   using D = Desc<Q>;
   using T = DynTraits<DYN>;
-  if constexpr (DYN == DYN_BGK && sizeof(R) == 4) {
-    collide_bgk_f32<Q>(f, p.omega, rhoOut, uSqrOut);
+  if constexpr (DYN != DYN_CONST_RHO && sizeof(R) == 4) {
+    collide_f32<Q, DYN>(f, p, rhoOut, uSqrOut);
     return;
   }
   R rho, u[3];
@@ -245,7 +432,7 @@ __device__ __forceinline__ void collide(R (&f)[Q], const CollisionParams<R>& p, 
   }
 
   if constexpr (T::trt) {
-    const R omega2 = R(1) / (p.magic / (R(1) / omega - R(0.5)) + R(0.5));
+    const R omega2 = p.omega2;
     // pairs (i, opp(i)) for i = 1 .. q/2, plus the rest population
     {
       const R feq0 = equilibrium<Q, 0>(rho, u, uSqr);
@@ -268,32 +455,12 @@ __device__ __forceinline__ void collide(R (&f)[Q], const CollisionParams<R>& p, 
       f[i] = fi - (omega * (fpi - epi) + omega2 * (fmi - emi));
       f[j] = fj - (omega * (fpj - epj) + omega2 * (fmj - emj));
     });
-  } else if constexpr (sizeof(R) == 8) {
+  } else {
     const R keep = R(1) - omega;
     static_for<Q>([&](auto I) {
       const R feq = equilibrium<Q, I>(rho, u, uSqr);
       f[I] *= keep;
       f[I] += omega * feq;
-    });
-  } else {
-    // float: opposite directions share t_i and |c_i . u|, so their equilibria are
-    // sym +- asym with sym = rho t (1 - 1.5 u^2 + 4.5 (c.u)^2) - t and asym = 3 rho t (c.u)
-    const R keep = R(1) - omega;
-    const R base = R(1) - R(1.5) * uSqr;
-    {
-      constexpr R t0 = weight<Q, R>(0);
-      f[0] = __fmaf_rn(omega, __fmaf_rn(rho * t0, base, -t0), f[0] * keep);
-    }
-    static_for<Q / 2>([&](auto K) {
-      constexpr int i = K + 1;
-      constexpr int j = D::OPP[i];
-      constexpr R t = weight<Q, R>(i);
-      const R cu = c_dot<Q, i>(u);
-      const R rt = rho * t;
-      const R sym = __fmaf_rn(rt, __fmaf_rn(R(4.5) * cu, cu, base), -t);
-      const R asym = (rho * R(3 * t)) * cu;
-      f[i] = __fmaf_rn(omega, sym + asym, f[i] * keep);
-      f[j] = __fmaf_rn(omega, sym - asym, f[j] * keep);
     });
   }
 
@@ -313,78 +480,6 @@ __device__ __forceinline__ void collide(R (&f)[Q], const CollisionParams<R>& p, 
   }
   rhoOut = rho;
   uSqrOut = uSqr;
-}
-
-// ---- two cells at once: packed FP32 pairs (sm_100 f32x2 arithmetic) ------------------------
-// Each packed operation rounds every lane exactly as the scalar operation does, so a pair of
-// cells computed here gets the same bits as two calls of the scalar float path below: the
-// operation sequence of collide<Q, float, DYN_BGK> is kept step for step.
-// The pairs are CUDA's float2 and the operations its sm_100 packed intrinsics, whose rounding per
-// component is that of __fadd_rn, __fmul_rn and __fmaf_rn; the compiler keeps a pair in a
-// register pair instead of packing two floats around every operation.
-using F2 = float2;
-__device__ __forceinline__ F2 f2(float v) { return make_float2(v, v); }
-__device__ __forceinline__ F2 add2(F2 a, F2 b) { return __fadd2_rn(a, b); }
-// a - b with one rounding, as __fsub_rn: b * (-1) is exact, so the fused form rounds a + (-b) once
-__device__ __forceinline__ F2 sub2(F2 a, F2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
-__device__ __forceinline__ F2 mul2(F2 a, F2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) { return __ffma2_rn(a, b, c); }
-
-// BGK collision of two cells (f[k][i], k = 0, 1) in place: collide_bgk_f32 on pairs, the same
-// operation sequence (no product ever meets a separate add, so no contraction can differ).
-template <int Q>
-__device__ __forceinline__ void collide_bgk_x2(float (&f)[2][Q], float omega, float (&rhoOut)[2], float (&usqOut)[2]) {
-  using D = Desc<Q>;
-  F2 g[Q];
-  static_for<Q>([&](auto I) { g[I] = F2{f[0][I], f[1][I]}; });
-  F2 rho = f2(0.f);
-  static_for<Q>([&](auto I) { rho = add2(rho, g[I]); });
-  rho = add2(rho, f2(1.f));
-  F2 j[3] = {f2(0.f), f2(0.f), f2(0.f)};
-  static_for<Q>([&](auto I) {
-    static_for<D::d>([&](auto A) {
-      constexpr int c = D::C[I][A];
-      if constexpr (c == 1) j[A] = add2(j[A], g[I]);
-      else if constexpr (c == -1) j[A] = sub2(j[A], g[I]);
-    });
-  });
-  const F2 inv{1.f / rho.x, 1.f / rho.y};
-  F2 u[3];
-  static_for<D::d>([&](auto A) { u[A] = mul2(j[A], inv); });
-  F2 uSqr = mul2(u[0], u[0]);
-  static_for<D::d - 1>([&](auto A) { uSqr = fma2(u[A + 1], u[A + 1], uSqr); });
-  const F2 w = f2(omega);
-  const F2 keep = f2(1.f - omega);
-  const F2 base = fma2(f2(-1.5f), uSqr, f2(1.f));
-  {
-    constexpr float t0 = weight<Q, float>(0);
-    g[0] = fma2(w, fma2(mul2(rho, f2(t0)), base, f2(-t0)), mul2(g[0], keep));
-  }
-  static_for<Q / 2>([&](auto K) {
-    constexpr int i = K + 1;
-    constexpr int jj = D::OPP[i];
-    constexpr float t = weight<Q, float>(i);
-    F2 cj = f2(0.f);
-    static_for<D::d>([&](auto A) {
-      constexpr int c = D::C[i][A];
-      if constexpr (c == 1) cj = add2(cj, j[A]);
-      else if constexpr (c == -1) cj = sub2(cj, j[A]);
-    });
-    const F2 cu = mul2(cj, inv);
-    const F2 sym = fma2(mul2(rho, f2(t)), fma2(mul2(f2(4.5f), cu), cu, base), f2(-t));
-    const F2 r3t = mul2(rho, f2(3 * t));
-    const F2 plus = fma2(r3t, cu, sym), minus = fma2(F2{-r3t.x, -r3t.y}, cu, sym);
-    g[i] = fma2(w, plus, mul2(g[i], keep));
-    g[jj] = fma2(w, minus, mul2(g[jj], keep));
-  });
-  static_for<Q>([&](auto I) {
-    f[0][I] = g[I].x;
-    f[1][I] = g[I].y;
-  });
-  rhoOut[0] = rho.x;
-  rhoOut[1] = rho.y;
-  usqOut[0] = uSqr.x;
-  usqOut[1] = uSqr.y;
 }
 
 template <int Q, typename R>

@@ -62,6 +62,7 @@ struct EnsLattice {
   int64_t steps, maxSteps;
   double tol, residual;
   float omega, magic;
+  float relax[4];            // Relaxation::set of them
   float delta[kMaxQ];        // wall term of the links leaving through the moving lid
   uint32_t shift[2][kMaxQ];  // column shifts, double-buffered by global step parity
 };
@@ -242,7 +243,8 @@ __device__ __forceinline__ void ensemble_tiles(const EnsArgs& a, int par, int nT
     S* pop = static_cast<S*>(L->pop);
     CollisionParams<R> cp;
     cp.omega = R(L->omega);
-    cp.magic = R(L->magic);
+    cp.omega2 = trt_omega2(R(L->omega), R(L->magic));
+    for (int k = 0; k < 4; ++k) cp.relax[k] = L->relax[k];
     cp.smagorinsky = R(0);
     cp.force[0] = cp.force[1] = cp.force[2] = R(0);
     cp.avgSrc = nullptr;
@@ -978,6 +980,7 @@ int lbx_ensemble_admit(lbx_ensemble E, const lbx_ensemble_request* req, int32_t*
   L.residual = INFINITY;
   L.omega = float(req->params.omega);
   L.magic = float(req->params.magic);
+  Relaxation::set(E->q, L.omega, L.magic, L.dynamics == LBX_TRT, L.relax);
   for (int k = 0; k < E->q; ++k) {
     const int* c = E->q == 19 ? Desc<19>::C[k] : Desc<27>::C[k];
     const double w = E->q == 19 ? double(Desc<19>::WN[k]) / Desc<19>::WD[k] : double(Desc<27>::WN[k]) / Desc<27>::WD[k];

@@ -767,7 +767,7 @@ __global__ void __launch_bounds__(WsCfg<Q, S>::THREADS, WsCfg<Q, S>::BLOCKS) k_c
   constexpr int ES = C::ES, BT = C::BT, NS = C::NS;
   constexpr int COL = C::COL_BYTES / ES;      // elements per column buffer
   constexpr int NCT = 32 * C::CONSUMER_WARPS;  // consumer threads
-  constexpr bool PACKED = sizeof(R) == 4 && sizeof(S) == 2 && DYN == DYN_BGK;
+  constexpr bool PACKED = sizeof(R) == 4 && sizeof(S) == 2 && DYN != DYN_CONST_RHO;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw + NS * C::STAGE_BYTES);
   uint64_t* empty = full + NS;
@@ -909,7 +909,7 @@ __global__ void __launch_bounds__(WsCfg<Q, S>::THREADS, WsCfg<Q, S>::BLOCKS) k_c
         if constexpr (PACKED) {
           if (bulk[0] && bulk[1]) {
             float rr[2], uu[2];
-            collide_bgk_x2<Q>(f, p.omega, rr, uu);
+            collide_x2<Q, DYN>(f, p, rr, uu);
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
               accRho += double(rr[c]);
@@ -1129,25 +1129,28 @@ __global__ void __launch_bounds__(256, StepOccupancy<Q, S, K>::blocks) k_collide
 #pragma unroll
     for (int k = 0; k < K; ++k)
       static_for<Q>([&](auto I) { f[k][I] = act[k] ? Storage<S>::load(&raw[k][I]) : R(0); });
-    // pairs of bulk BGK cells of a 16-bit form: one packed (f32x2) collision per pair, the same
-    // bits as two scalar ones.  The 16-bit forms are limited by instruction issue, where the
-    // packed form halves the collision's arithmetic; the FP32 form waits on HBM, and there the
-    // packed form's extra registers cost more than they save.
-    constexpr bool PACKED = K >= 2 && sizeof(R) == 4 && sizeof(S) == 2 && DYN == DYN_BGK;
+    // pairs of cells: one packed (f32x2) collision, the same bits as two scalar ones.  A cell of the
+    // pair that is not a bulk cell was not loaded and is not stored, so what the pair makes of its
+    // zeros is dropped; only a bounce-back cell, which keeps its own populations, sends its pair to
+    // the scalar path.
+    constexpr bool PACKED = K >= 2 && sizeof(R) == 4 && DYN != DYN_CONST_RHO;
+    auto count = [&](R rho, R usq) {
+      accRho += double(rho);
+      accUsq += double(usq);
+      accMax = fmax(accMax, double(usq));
+      ++accCount;
+    };
 #pragma unroll
     for (int pr = 0; pr < (K + 1) / 2; ++pr) {
       const int k0 = 2 * pr, k1 = 2 * pr + 1;
       bool packedDone = false;
       if constexpr (PACKED) {
-        if (k1 < K && bulk_kind(kinds[k0]) && bulk_kind(kinds[k1])) {
+        if (k1 < K && kinds[k0] != 2 && kinds[k1] != 2) {
           float rr[2], uu[2];
-          collide_bgk_x2<Q>(*reinterpret_cast<float(*)[2][Q]>(&f[k0]), p.omega, rr, uu);
-#pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            accRho += double(rr[k]);
-            accUsq += double(uu[k]);
-            accMax = fmax(accMax, double(uu[k]));
-            ++accCount;
+          collide_x2<Q, DYN>(*reinterpret_cast<float(*)[2][Q]>(&f[k0]), p, rr, uu);
+          if (statPart) {
+            if (bulk_kind(kinds[k0])) count(rr[0], uu[0]);
+            if (bulk_kind(kinds[k1])) count(rr[1], uu[1]);
           }
           packedDone = true;
         }
@@ -1159,10 +1162,7 @@ __global__ void __launch_bounds__(256, StepOccupancy<Q, S, K>::blocks) k_collide
           if (bulk_kind(kinds[k])) {
             R rho, usq;
             collide<Q, R, DYN>(f[k], p, rho, usq);
-            accRho += double(rho);
-            accUsq += double(usq);
-            accMax = fmax(accMax, double(usq));
-            ++accCount;
+            if (statPart) count(rho, usq);
           } else if (kinds[k] == 2) {
             revert<Q, R>(f[k]);
           }
@@ -2357,11 +2357,12 @@ inline Shifts<Q> shifts_of(const LaunchArgs& a) {
   return s;
 }
 
-template <typename R>
+template <int Q, typename R>
 inline CollisionParams<R> params_of(const LaunchArgs& a) {
   CollisionParams<R> p;
   p.omega = R(a.omega);
-  p.magic = R(a.magic);
+  p.omega2 = trt_omega2(R(a.omega), R(a.magic));
+  Relaxation::set(Q, float(a.omega), float(a.magic), a.dynamics == DYN_TRT, p.relax);
   p.smagorinsky = R(a.smagorinsky);
   for (int k = 0; k < 3; ++k) p.force[k] = R(a.force[k]);
   p.avgSrc = a.avgSrc;
@@ -2377,7 +2378,7 @@ cudaError_t launch_step_dyn(const LaunchArgs& a, cudaStream_t stream) {
   using R = typename Storage<S>::R;
   const Geometry& g = a.g;
   const auto sh = shifts_of<Q>(a);
-  const auto p = params_of<R>(a);
+  const auto p = params_of<Q, R>(a);
   S* pop = static_cast<S*>(a.pop);
   int64_t nblocks = 0;
   if (a.kernel == 0) {
@@ -2476,7 +2477,9 @@ cudaError_t launch_step_dyn(const LaunchArgs& a, cudaStream_t stream) {
     for (int c = 0; c < 3; ++c) {
       cls.p[c] = p;
       cls.p[c].omega = R(a.classParam[c][0]);
-      cls.p[c].magic = R(a.classParam[c][1]);
+      cls.p[c].omega2 = trt_omega2(R(a.classParam[c][0]), R(a.classParam[c][1]));
+      const bool trt = (a.classDyn[c] ? a.classDyn[c] : a.dynamics) == DYN_TRT;
+      Relaxation::set(Q, float(a.classParam[c][0]), float(a.classParam[c][1]), trt, cls.p[c].relax);
       cls.p[c].smagorinsky = R(a.classParam[c][2]);
       for (int k = 0; k < 3; ++k) cls.p[c].force[k] = R(a.classParam[c][3 + k]);
     }

@@ -1,0 +1,59 @@
+"""Paths that a step can take give the same bits: the packed two-cell collision against the scalar
+one, for every dynamics, on lattices whose cell pairs mix bulk cells with solid and bounce-back ones."""
+import numpy as np
+import pytest
+
+from openlb_b200 import lbx
+
+pytestmark = pytest.mark.gpu
+
+DYNAMICS = ["bgk", "trt", "smagorinsky_bgk", "forced_bgk", "smagorinsky_forced_bgk"]
+
+
+def lattice(q, core, periodic, storage, dynamics, solid=0.0, bounce=0.0, lid=None, seed=11):
+    """A lattice with random populations, a share `solid` of cells without dynamics behind halfway
+    bounce-back links, a share `bounce` of bounce-back cells, and with `lid` a moving top layer."""
+    rng = np.random.default_rng(seed)
+    lat = lbx.BlockLattice(q, core, periodic, storage)
+    lat.define_dynamics(dynamics, omega=1.35, magic=0.2, smagorinsky=0.14, force=(1e-4, -3e-5, 2e-5))
+    full = lat.core
+    mat = np.ones(full, np.int32)
+    if solid:
+        mat[rng.random(full) < solid] = 2
+    if lid is not None:
+        mat[:, -1, :] = 3
+    ids = np.where(mat == 1, lbx.CELL_BULK, lbx.CELL_NONE)
+    if bounce:
+        ids[(rng.random(full) < bounce) & (mat == 1)] = lbx.CELL_BOUNCE_BACK
+    if solid or bounce or lid is not None:
+        lat.set_cell_dynamics(ids.astype(np.uint8))
+    if solid or lid is not None:
+        fluid = np.where(ids == lbx.CELL_BULK, 1, np.where(mat == 1, 4, mat)).astype(np.int32)
+        lat.set_bouzidi_boundary(fluid, 1, (2, 3), wall_velocity=[(0, 0, 0), lid] if lid is not None else None)
+    lat.set_populations((rng.random((q, lat.n_core)) - 0.5) * 1e-2)
+    return lat
+
+
+def populations(lat):
+    out = lat.get_populations(np.float64)
+    lat.close()
+    return out
+
+
+@pytest.mark.parametrize("dynamics", DYNAMICS)
+@pytest.mark.parametrize("q,core,storage", [(19, (5, 6, 67), "f32"), (27, (4, 5, 97), "f16dev"),
+                                            (9, (7, 130), "f32"), (19, (3, 4, 33), "bf16dev")])
+def test_packed_pairs_match_single_cells(dynamics, q, core, storage):
+    for kw in ({}, {"solid": 0.3}, {"bounce": 0.1, "solid": 0.1}):
+        ref = None
+        for cells in (1, 2):
+            lat = lattice(q, core, (1, 1, 1 if q != 9 else 0), storage, dynamics, **kw)
+            lat.set_launch_config(2, 32, 4, cells)
+            for _ in range(6):
+                lat.collide_and_stream(1)
+            f = populations(lat)
+            assert np.isfinite(f).all()
+            if ref is None:
+                ref = f
+            else:
+                assert np.array_equal(ref, f)
