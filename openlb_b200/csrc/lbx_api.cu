@@ -9,6 +9,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -133,8 +134,9 @@ struct lbx_lattice_s {
   std::vector<uint32_t> linkHostCell;
   std::vector<uint8_t> linkHostDir;
   std::vector<double> linkHostDelta;
-  // resting links fused into the K-cells step kernel (one direction bit per padded cell) and the
-  // links the link kernel still applies after that kernel (moving walls, unusual neighbours)
+  // links fused into the K-cells step kernel (one direction bit per padded cell, and the class of
+  // the cell's moving-wall terms) and the links the link kernel still applies after that kernel
+  // (unusual neighbours, more wall terms than there are classes)
   // bounce-back cells with a wall velocity (lbx_set_bounce_back_velocity): padded cells ascending
   // and {rho, u} per cell
   int64_t nBbv = 0;
@@ -145,6 +147,7 @@ struct lbx_lattice_s {
   // velocity list, or -1 (the boundary kernels' neighbour lookups); null without such cells
   int32_t* bIdx = nullptr;
   uint32_t* linkMask = nullptr;
+  void* wallDelta = nullptr;  // [kWallClasses][q] wall terms, null when every fused wall is at rest
   uint32_t* restCell = nullptr;
   uint8_t* restDir = nullptr;
   void* restDelta = nullptr;
@@ -232,6 +235,7 @@ LaunchArgs args_of(const lbx_lattice_s* L) {
   a.fdMom = L->fdMom;
   a.nFdCorners = L->nFdCorners;
   a.linkMask = groups_kernel(L->kernel) ? L->linkMask : nullptr;
+  a.wallDelta = L->wallDelta;
   a.nBbv = L->nBbv;
   a.bbvCell = L->bbvCell;
   a.bbvValue = L->bbvValue;
@@ -559,10 +563,6 @@ bool device_ok(int device, std::string& why) {
 }
 
 
-// Composes the device cell map from the map as set and the links, and splits the links: a link
-// from a bulk cell (x_b, k) towards a cell without dynamics, at rest (no wall term), is fused
-// into the K-cells step kernel (bit k of linkMask[x_b], x_b marked kCellBulkLinked); every other
-// link stays with the link kernel, which with the other kernel variants applies all links.
 // The per-cell boundary index (lbx_lattice_s::bIdx) from the two boundary lists.
 int refresh_boundary_index(lbx_lattice_s* L) {
   cudaFree(L->bIdx);
@@ -576,15 +576,23 @@ int refresh_boundary_index(lbx_lattice_s* L) {
   return LBX_OK;
 }
 
+// Composes the device cell map from the map as set and the links, and splits the links: a link
+// from a bulk cell (x_b, k) towards a cell without dynamics is fused into the K-cells step kernel
+// (bit k of linkMask[x_b], x_b marked kCellBulkLinked).  The wall terms of such a cell, by
+// direction, are its class; a moving lid has a handful (its rows, edges and corners).  Every other
+// link, and the moving ones of cells beyond the last class, stays with the link kernel, which with
+// the other kernel variants applies all links.
 int refresh_cell_map(lbx_lattice_s* L) {
   ++L->mapVersion;
   if (int rc = refresh_boundary_index(L)) return rc;
   const bool need = !L->hostMap.empty() || L->nLinks > 0;
   cudaFree(L->linkMask);
+  cudaFree(L->wallDelta);
   cudaFree(L->restCell);
   cudaFree(L->restDir);
   cudaFree(L->restDelta);
   L->linkMask = nullptr;
+  L->wallDelta = nullptr;
   L->restCell = nullptr;
   L->restDir = nullptr;
   L->restDelta = nullptr;
@@ -608,6 +616,8 @@ int refresh_cell_map(lbx_lattice_s* L) {
     mask.assign(static_cast<size_t>(L->n), 0u);
     const Geometry g = geometry_of(L);
     const int64_t ext[3] = {g.nx, g.ny, g.nz};
+    std::vector<uint8_t> fuse(L->linkHostCell.size(), 0);
+    std::map<uint32_t, std::vector<double>> moving;  // per cell: wall terms by direction
     for (size_t l = 0; l < L->linkHostCell.size(); ++l) {
       const uint32_t src = L->linkHostCell[l];
       const int k = L->linkHostDir[l];
@@ -627,15 +637,43 @@ int refresh_cell_map(lbx_lattice_s* L) {
         }
       }
       const int64_t tgt = inside ? (p[0] + 1) * g.sx + (p[1] + 1) * g.sy + (p[2] + g.pz) : -1;
-      const bool fuse = L->linkHostDelta[l] == 0.0 && map[src] == LBX_CELL_BULK && tgt >= 0 &&
-                        map[size_t(tgt)] == LBX_CELL_NONE;
-      if (fuse) {
-        mask[src] |= 1u << k;
+      fuse[l] = map[src] == LBX_CELL_BULK && tgt >= 0 && map[size_t(tgt)] == LBX_CELL_NONE;
+      if (fuse[l] && L->linkHostDelta[l] != 0.0) {
+        std::vector<double>& terms = moving[src];
+        terms.resize(size_t(L->q), 0.0);
+        terms[size_t(k)] = L->linkHostDelta[l];
+      }
+    }
+    std::map<std::vector<double>, uint32_t> classes;
+    for (const auto& cell : moving)
+      if (classes.size() + 1 < size_t(kWallClasses)) classes.emplace(cell.second, uint32_t(classes.size() + 1));
+    for (size_t l = 0; l < L->linkHostCell.size(); ++l) {
+      const uint32_t src = L->linkHostCell[l];
+      bool fused = fuse[l] != 0;
+      if (fused && L->linkHostDelta[l] != 0.0) {
+        const auto c = classes.find(moving[src]);
+        fused = c != classes.end();
+        if (fused) mask[src] |= c->second << kWallShift;
+      }
+      if (fused) {
+        mask[src] |= 1u << L->linkHostDir[l];
       } else {
         rc.push_back(src);
-        rd.push_back(uint8_t(k));
+        rd.push_back(L->linkHostDir[l]);
         rdelta.push_back(L->linkHostDelta[l]);
         restWall = restWall || L->linkHostDelta[l] != 0.0;
+      }
+    }
+    if (!classes.empty()) {
+      std::vector<double> terms(size_t(kWallClasses) * size_t(L->q), 0.0);
+      for (const auto& c : classes) std::copy(c.first.begin(), c.first.end(), terms.begin() + c.second * size_t(L->q));
+      if (L->storage == LBX_F64) {
+        LBX_CUDA_TRY(cudaMalloc(&L->wallDelta, terms.size() * sizeof(double)));
+        LBX_CUDA_TRY(cudaMemcpy(L->wallDelta, terms.data(), terms.size() * sizeof(double), cudaMemcpyHostToDevice));
+      } else {
+        const std::vector<float> tf(terms.begin(), terms.end());
+        LBX_CUDA_TRY(cudaMalloc(&L->wallDelta, tf.size() * sizeof(float)));
+        LBX_CUDA_TRY(cudaMemcpy(L->wallDelta, tf.data(), tf.size() * sizeof(float), cudaMemcpyHostToDevice));
       }
     }
     bool any = false;
@@ -995,6 +1033,7 @@ int lbx_lattice_destroy(lbx_lattice L) {
   cudaFree(L->linkDelta);
   cudaFree(L->linkGroup);
   cudaFree(L->linkMask);
+  cudaFree(L->wallDelta);
   cudaFree(L->restCell);
   cudaFree(L->restDir);
   cudaFree(L->restDelta);

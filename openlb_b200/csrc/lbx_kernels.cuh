@@ -73,11 +73,14 @@ __device__ __forceinline__ int64_t wrap_add(int64_t a, int64_t s, int64_t n) {
 
 // Cell kinds of the device cell map: the public ids (0 no dynamics, 1 bulk, 2 bounce-back,
 // 3 velocity / pressure boundary, 4 bounce-back with a wall velocity) plus 7, a bulk cell some of
-// whose populations leave towards a resting halfway bounce-back wall; the K-cells step kernel
+// whose populations leave towards a halfway bounce-back wall; the K-cells step kernel
 // writes those populations back into the cell's opposite slots itself (see
 // k_collide_stream_groups), the other kernels treat 7 as 1.  Kinds 3 and 4 are collided by their
 // own kernels after the bulk kernel, which neither loads nor stores them.
 constexpr uint8_t kCellBulkLinked = 7;
+// linkMask of such a cell: bit k for a link along direction k, and above the directions the cell's
+// class of moving-wall terms (0: every wall at rest), a row of LaunchArgs::wallDelta
+constexpr int kWallShift = 27, kWallClasses = 32;
 constexpr uint8_t kCellBounceBackVelocity = 4;
 // 8, 9, 10: bulk cells colliding with the parameters of class 1, 2, 3 (lbx_set_dynamics_class;
 // stepped by the one-cell-per-thread kernel only, which a lattice with classes always uses)
@@ -998,6 +1001,17 @@ template <> struct StepOccupancy<19, __nv_bfloat16, 4> { static constexpr int bl
 template <> struct StepOccupancy<9, __half, 4> { static constexpr int blocks = 2; };
 template <> struct StepOccupancy<9, __nv_bfloat16, 4> { static constexpr int blocks = 2; };
 
+// What a wall link sends back of population i: the stored value of what the cell sent, less the
+// wall's term where the wall moves (`wall`: the terms of the cell's class by direction, null for a
+// wall at rest), as the link kernel reads and writes it after the stream.
+template <typename S, typename R>
+__device__ __forceinline__ R bounced(R f, const R* __restrict__ wall, int i) {
+  if (!wall) return f;
+  S stored;
+  Storage<S>::store(&stored, f);
+  return Storage<S>::load(&stored) - wall[i];
+}
+
 // Load of one stored population of a 16-bit form with an L2 prefetch-size hint of 256 bytes: a
 // warp-wide load reads 64 bytes of a column, and the hint lets L2 fetch the following warps'
 // bytes of the same column with the same DRAM access.  (The line stays in L1: the second cell of
@@ -1020,6 +1034,7 @@ __global__ void __launch_bounds__(256, StepOccupancy<Q, S, K>::blocks) k_collide
                                                                CollisionParams<typename Storage<S>::R> p,
                                                                const uint8_t* __restrict__ cellDyn,
                                                                const uint32_t* __restrict__ linkMask,
+                                                               const typename Storage<S>::R* __restrict__ wallDelta,
                                                                double* __restrict__ statPart, int ahead) {
   using R = typename Storage<S>::R;
   using D = Desc<Q>;
@@ -1227,29 +1242,31 @@ __global__ void __launch_bounds__(256, StepOccupancy<Q, S, K>::blocks) k_collide
         });
       }
     }
-    // resting halfway bounce-back (BouzidiPostProcessor with q = 1/2 and a wall at rest,
-    // boundary/setBouzidiBoundary.h:48-77), fused into the store: a population f_k that leaves the
-    // cell towards a solid neighbour x_s = x_b + c_k is also written into the slot of x_s's
-    // opposite population, which the rotation of this step carries into f_opp(k)(x_b) -- the value
-    // the link kernel would copy there after the stream.  The solid cell has no dynamics, so no
+    // halfway bounce-back (BouzidiPostProcessor with q = 1/2, boundary/setBouzidiBoundary.h:48-77,
+    // 129-162), fused into the store: a population f_k that leaves the cell towards a solid
+    // neighbour x_s = x_b + c_k is also written, less the term of a moving wall, into the slot of
+    // x_s's opposite population, which the rotation of this step carries into f_opp(k)(x_b) -- the
+    // value the link kernel would put there after the stream.  The solid cell has no dynamics, so no
     // other thread writes that slot (cells without dynamics make no stores, ghost ones included).
     if (MAPPED && linkMask) {
 #pragma unroll
       for (int k = 0; k < K; ++k) {
         if (kinds[k] != kCellBulkLinked) continue;
         const uint32_t mk = linkMask[n0 + W * k];
+        const R* wall = (mk >> kWallShift) ? wallDelta + int(mk >> kWallShift) * Q : nullptr;
         static_for<Q>([&](auto I) {
           if ((mk >> int(I)) & 1u) {
             constexpr int O = D::OPP[I];
             const int32_t off = int32_t(D::C[I][0] * g.sx + D::C[I][1] * g.sy + D::C[I][2]);
             S* col = static_cast<S*>(cols.base[O]);
             const uint32_t slot = n0 + W * k + uint32_t(off);
+            const R v = bounced<S>(f[k][I], wall, I);
             if constexpr (DOUBLED) {
-              Storage<S>::store(col + slot, f[k][I]);
+              Storage<S>::store(col + slot, v);
             } else {
               uint32_t idx = slot + cols.s[O];
               idx = idx >= P ? idx - P : idx;
-              Storage<S>::store(col + idx, f[k][I]);
+              Storage<S>::store(col + idx, v);
             }
           }
         });
@@ -2280,7 +2297,8 @@ struct LaunchArgs {
   const double* fdValue;     // 4 imposed values per cell
   double* fdMom;             // 7 doubles per cell of scratch (k_fd_momenta)
   int64_t nFdCorners;        // how many of them are corners (regularised in a second pass)
-  const uint32_t* linkMask;  // per padded cell: directions of resting bounce-back links (kind 7 cells)
+  const uint32_t* linkMask;  // per padded cell: directions of fused bounce-back links (kind 7 cells)
+  const void* wallDelta;     // wall terms of their classes, [kWallClasses][Q] (null: every wall at rest)
   int64_t nBbv;              // bounce-back cells with a wall velocity
   const uint32_t* bbvCell;   // their padded indices
   const double* bbvValue;    // {rho, u} per cell
@@ -2508,7 +2526,8 @@ cudaError_t launch_step_dyn(const LaunchArgs& a, cudaStream_t stream) {
       int ahead = 0;
       if constexpr (decltype(doubled)::value)
         if (a.kernel == 5) ahead = l2_ahead_blocks(kern, int(block.x * block.y), aheadCache);
-      kern<<<grid, block, 0, stream>>>(cols, g, p, a.cellDyn, a.linkMask, part, ahead);
+      kern<<<grid, block, 0, stream>>>(cols, g, p, a.cellDyn, a.linkMask, static_cast<const R*>(a.wallDelta), part,
+                                       ahead);
     };
     auto go_k = [&](auto kk) {
       if (a.doubled) {

@@ -57,3 +57,35 @@ def test_packed_pairs_match_single_cells(dynamics, q, core, storage):
                 ref = f
             else:
                 assert np.array_equal(ref, f)
+
+
+@pytest.mark.parametrize("storage", ["f64", "f32", "f16dev"])
+@pytest.mark.parametrize("q,core", [(19, (9, 8, 34)), (27, (6, 7, 33)), (9, (20, 37))])
+def test_fused_moving_walls_match_the_link_kernel(q, core, storage):
+    """Links of a moving wall, fused into the step's store, against the link kernel (variant 1); with
+    a wall velocity that differs from cell to cell there are more wall terms than classes, and the
+    step fuses some and leaves the others."""
+    ref = None
+    for variant, block in ((1, (32, 8)), (2, (32, 8)), (2, (64, 4))):
+        lat = lattice(q, core, (0, 0, 0), storage, "bgk", solid=0.1, lid=(0.05, 0.0, 0.01))
+        lat.set_launch_config(variant, *block, 1)
+        lat.post_process()
+        for _ in range(5):
+            lat.collide_and_stream(1)
+        f = populations(lat)
+        ref = f if ref is None else ref
+        assert np.array_equal(ref, f)
+    ref = None
+    for variant in (1, 2):
+        lat = lattice(q, core, (0, 0, 0), storage, "bgk", lid=(0.05, 0.0, 0.01))
+        mat = np.ones(lat.core, np.int32)
+        mat[:, -1, :] = 3
+        cells, dirs, wall = lbx.build_bouzidi_links(q, lat.core, mat, 1, (3,), [(1.0, 0.0, 0.0)])
+        wall = wall * (0.02 + 1e-4 * np.arange(len(cells)))
+        lat.set_bouzidi_links(cells, dirs, wall)
+        lat.set_launch_config(variant, 32, 8, 1)
+        for _ in range(5):
+            lat.collide_and_stream(1)
+        f = populations(lat)
+        ref = f if ref is None else ref
+        assert np.array_equal(ref, f)
