@@ -164,9 +164,9 @@ __device__ __forceinline__ R smagorinsky_omega(const R (&f)[Q], R rho, const R (
 // ---- FP32 collisions, one cell or two at once ------------------------------------------------
 // The arithmetic of the FP32 and 16-bit forms, on a float (one cell) or a float2 (a pair of cells, on
 // the packed two-lane instructions of sm_100).  Every operation is an explicitly rounded add,
-// multiply or fused multiply-add, so nothing is left for the compiler to contract, and a lane of a
-// pair gets the bits of a single cell: CUDA's packed intrinsics round each component as __fadd_rn,
-// __fmul_rn and __fmaf_rn do.
+// multiply or fused multiply-add, and no product is the operand of a separate add (a packed pair of
+// those does get fused), so a lane of a pair gets the bits of a single cell: CUDA's packed
+// intrinsics round each component as __fadd_rn, __fmul_rn and __fmaf_rn do.
 using F2 = float2;
 __device__ __forceinline__ float vadd(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float vsub(float a, float b) { return __fsub_rn(a, b); }
@@ -271,14 +271,13 @@ __device__ __forceinline__ void collide_f32(V (&f)[Q], const CollisionParams<flo
   if constexpr (T::smagorinsky) {
     // Pi^neq with the unforced momentum j; n2 = sum of its squared components
     V n2 = vset<V>(0.f);
-    const V third = vmul(delta, vset<V>(-1.f / 3.f));
     static_for<D::d>([&](auto A) {
       const V ja = vmul(j[A], inv);
       static_for<D::d>([&](auto B) {
         if constexpr (B >= A) {
           constexpr int ip = A * D::d - (A * (A - 1)) / 2 + (B - A);
           V s = vfma(vmul(ja, vset<V>(-1.f)), j[B], pi[ip]);
-          if constexpr (A == B) s = vadd(s, third);
+          if constexpr (A == B) s = vfma(delta, vset<V>(-1.f / 3.f), s);
           if constexpr (T::forced) {
             if constexpr (A == B) {
               s = vfma(vset<V>(p.force[A]), j[A], s);

@@ -51,6 +51,31 @@ template <> struct Storage<__nv_bfloat16> {
   static __device__ __forceinline__ void store(__nv_bfloat16* p, R v) { *p = __float2bfloat16_rn(v); }
 };
 
+// ---- launches that follow one another -----------------------------------------------------
+// The kernels of a step are launched with programmatic stream serialization: each lets the next
+// one's blocks start while its own last ones run (chain_next, at its top) and waits for the one
+// before, its stores included, before it touches what that may have written (chain_wait).  Every
+// such kernel waits in every thread, so a kernel's completion implies that of all before it.  What
+// is set up before the steps (cell kinds, link masks, boundary lists) may be read ahead of the wait;
+// what a kernel of the chain writes is not passed as a __restrict__ pointer, whose loads the compiler
+// may move across the wait.
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename... P, typename... A>
+cudaError_t launch_chained(void (*kern)(P...), dim3 grid, dim3 block, cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 // ---- geometry of one lattice as the kernels see it -------------------------------------
 struct Geometry {
   int64_t n;       // padded cells N (column length)
@@ -134,9 +159,11 @@ __device__ __forceinline__ void block_partial(double a, double b, double m, doub
 // partials t, t + 1024, ... in index order (eight loads in flight per thread), then a fixed
 // shared-memory tree.  One block of 1024 threads; the result depends only on the partials.
 constexpr int kFinalizeThreads = 1024;
-static __global__ void __launch_bounds__(kFinalizeThreads) k_stats_finalize(const double* __restrict__ part,
+static __global__ void __launch_bounds__(kFinalizeThreads) k_stats_finalize(const double* part,
                                                                            int64_t nblocks,
-                                                                           StatAcc* __restrict__ out) {
+                                                                           StatAcc* out) {
+  chain_next();
+  chain_wait();
   double a = 0, b = 0, m = 0, c = 0;
   constexpr int U = 8;
   int64_t i = threadIdx.x;
@@ -979,8 +1006,8 @@ struct ColumnBases {
 // 24-38 % faster than the compiler's 96-142 registers for TRT and Smagorinsky-forced BGK); at
 // six blocks its 27 values spill.
 template <int Q, typename S, int K> struct StepOccupancy { static constexpr int blocks = 1; };
-template <> struct StepOccupancy<19, __half, 1> { static constexpr int blocks = 6; };
-template <> struct StepOccupancy<19, __nv_bfloat16, 1> { static constexpr int blocks = 6; };
+template <> struct StepOccupancy<19, __half, 1> { static constexpr int blocks = 4; };
+template <> struct StepOccupancy<19, __nv_bfloat16, 1> { static constexpr int blocks = 4; };
 template <> struct StepOccupancy<27, float, 1> { static constexpr int blocks = 4; };
 // FP64 D3Q19, one cell per thread: three blocks (80 registers) run 2-3 % faster than the
 // compiler's choice (FP32 at two cells per thread is fastest with its own 96 registers)
@@ -1035,9 +1062,11 @@ __global__ void __launch_bounds__(256, StepOccupancy<Q, S, K>::blocks) k_collide
                                                                const uint8_t* __restrict__ cellDyn,
                                                                const uint32_t* __restrict__ linkMask,
                                                                const typename Storage<S>::R* __restrict__ wallDelta,
-                                                               double* __restrict__ statPart, int ahead) {
+                                                               double* __restrict__ statPart, int ahead, int flat,
+                                                               FlatDiv dv) {
   using R = typename Storage<S>::R;
   using D = Desc<Q>;
+  chain_next();
   const uint32_t P = uint32_t(g.n);
   // L2 prefetch of the block `ahead` blocks later in launch order (about one wave of resident
   // blocks on): its Q column runs, one cp.async.bulk.prefetch per column and row, issued by the
@@ -1076,33 +1105,54 @@ __global__ void __launch_bounds__(256, StepOccupancy<Q, S, K>::blocks) k_collide
       }
     }
   }
-  // The K cells of a thread lie a warp apart along the fastest axis (z0, z0 + 32, ...): each
+  // The K cells of a thread lie a warp apart along the fastest axis (n0, n0 + 32, ...): each
   // warp-wide load or store then covers one contiguous run of 32 cells, which a 16-bit column
   // moves in two full sectors, instead of every instruction touching twice the sectors it uses.
+  // Rows: a thread's cells lie in one row of the core.  Flat (`flat`): the threads run through the
+  // padded cells of a plane (2D: of the lattice), padding included, so that a row need not be a
+  // multiple of 32 K cells (groups_shape says when).
   constexpr int W = 32;
-  int x, y, z0, nvalid;  // nvalid: cells k < nvalid of this thread lie in the core
-  bool inside;
-  {
+  uint32_t n0;
+  int fz[K], sl[K];  // each cell's coordinate on the fastest axis, and on the one before it
+  bool ok[K];        // the cell lies in the core
+  bool inside = false;
+  if (flat) {
+    const uint32_t t = (blockIdx.x * blockDim.y + threadIdx.y) * blockDim.x + threadIdx.x;
+    const uint32_t q0 = (t / W) * (W * K) + t % W;
+    const uint32_t row = D::d == 3 ? uint32_t(g.sy) : uint32_t(g.sx);
+    const uint32_t m = D::d == 3 ? dv.my : dv.mx;
+    const int l = D::d == 3 ? dv.ly : dv.lx;
+    const int nf = D::d == 3 ? g.nz : g.ny, nrows = D::d == 3 ? g.ny : g.nx;
+    n0 = (D::d == 3 ? (blockIdx.z + 1u) * uint32_t(g.sx) + row : row) + 1u + q0;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const uint32_t q = q0 + uint32_t(W * k), r = (__umulhi(q, m) + q) >> l;
+      sl[k] = int(r);
+      fz[k] = int(q - r * row);
+      ok[k] = sl[k] < nrows && fz[k] < nf;
+      inside = inside || ok[k];
+    }
+  } else {
     const int gi = blockIdx.x * blockDim.x + threadIdx.x;
     const int m = blockIdx.y * blockDim.y + threadIdx.y;
-    z0 = (gi / W) * (W * K) + gi % W;
+    const int z0 = (gi / W) * (W * K) + gi % W;
     const int nf = D::d == 3 ? g.nz : g.ny;
-    if constexpr (D::d == 3) {
-      y = m; x = blockIdx.z;
-      inside = z0 < g.nz && y < g.ny;
-    } else {
-      x = m; y = 0;
-      inside = z0 < g.ny && x < g.nx;
+    const bool row = m < (D::d == 3 ? g.ny : g.nx);
+    // 3D: (x+1)*sx + (y+1)*sy + z0 + 1; 2D: the fast axis is y (sy = 1), z absent
+    n0 = D::d == 3 ? uint32_t((int(blockIdx.z) + 1) * g.sx + (m + 1) * g.sy + z0 + 1)
+                   : uint32_t((m + 1) * g.sx + z0 + 1);
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      sl[k] = m;
+      fz[k] = z0 + W * k;
+      ok[k] = row && fz[k] < nf;
     }
-    nvalid = (nf - z0 + W - 1) / W;
+    inside = ok[0];
   }
   double accRho = 0.0, accUsq = 0.0, accMax = 0.0;
   unsigned accCount = 0;
+  if (!inside) chain_wait();
   if (inside) {
-    // 3D: (x+1)*sx + (y+1)*sy + z0 + 1; 2D: the fast axis is y (sy = 1), z absent; cell k of
-    // the thread is n0 + W k
-    const uint32_t n0 = (D::d == 3) ? uint32_t((x + 1) * g.sx + (y + 1) * g.sy + z0 + 1)
-                                    : uint32_t((x + 1) * g.sx + z0 + 1);
     // the cell kinds first: a cell without dynamics is neither loaded nor stored, so the solid
     // part of a porous medium costs no population traffic (boundary cells of kinds 3 and 4 are
     // loaded and stored by their own kernels)
@@ -1113,13 +1163,14 @@ __global__ void __launch_bounds__(256, StepOccupancy<Q, S, K>::blocks) k_collide
 #pragma unroll
     for (int k = 0; k < K; ++k) {
       if constexpr (MAPPED) {
-        kinds[k] = (k < nvalid) ? cellDyn[n0 + W * k] : uint8_t(0);
+        kinds[k] = ok[k] ? cellDyn[n0 + W * k] : uint8_t(0);
         act[k] = stepped_kind(kinds[k]);
       } else {
-        kinds[k] = (k < nvalid) ? uint8_t(1) : uint8_t(0);
-        act[k] = k < nvalid;
+        kinds[k] = ok[k] ? uint8_t(1) : uint8_t(0);
+        act[k] = ok[k];
       }
     }
+    chain_wait();
     // raw loads next, all in straight-line code (the wrap is a select, not a branch), so every
     // load of the thread is in flight before the first value is used
     S raw[K][Q];
@@ -1190,8 +1241,6 @@ __global__ void __launch_bounds__(256, StepOccupancy<Q, S, K>::blocks) k_collide
     //  - other rows copy only what leaves across the fastest axis, which lands in the same
     //    row's ghost cell at the other end (n -+ nf).
     const int nf = D::d == 3 ? g.nz : g.ny;
-    const bool slowFace = ((g.pmask & 1) && (x == 0 || x == g.nx - 1)) ||
-                          (D::d == 3 && (g.pmask & 2) && (y == 0 || y == g.ny - 1));
     auto ghost_store = [&](auto I, int k, uint32_t slot) {
       S* col = static_cast<S*>(cols.base[I]);
       if constexpr (DOUBLED) {
@@ -1202,44 +1251,42 @@ __global__ void __launch_bounds__(256, StepOccupancy<Q, S, K>::blocks) k_collide
         Storage<S>::store(col + idx, f[k][I]);
       }
     };
-    if (slowFace) {
+    if (g.pmask) {
 #pragma unroll
       for (int k = 0; k < K; ++k) {
         // no dynamics: nothing to carry across (see linkMask); boundary cells: their own kernels
         if (!act[k]) continue;
-        const int cz0 = D::d == 3 ? z0 + W * k : 0;
-        const int cy0 = D::d == 3 ? y : z0 + W * k;
-        static_for<Q>([&](auto I) {
-          constexpr int cx = D::C[I][0], cy = D::C[I][1], cz = D::C[I][2];
-          int tx = x + cx, ty = cy0 + cy, tz = cz0 + cz;
-          bool crossed = false, lost = false;
-          if (tx < 0 || tx >= g.nx) { if (g.pmask & 1) { tx = tx < 0 ? tx + g.nx : tx - g.nx; crossed = true; } else lost = true; }
-          if (ty < 0 || ty >= g.ny) { if (g.pmask & 2) { ty = ty < 0 ? ty + g.ny : ty - g.ny; crossed = true; } else lost = true; }
-          if constexpr (D::d == 3) {
-            if (tz < 0 || tz >= g.nz) { if (g.pmask & 4) { tz = tz < 0 ? tz + g.nz : tz - g.nz; crossed = true; } else lost = true; }
-          }
-          if (crossed && !lost) {
-            const int64_t gn = int64_t(tx - cx + 1) * g.sx + int64_t(ty - cy + 1) * g.sy + (tz - cz + g.pz);
-            ghost_store(I, k, uint32_t(gn));
-          }
-        });
-      }
-    } else if (g.pmask & (D::d == 3 ? 4 : 2)) {
-#pragma unroll
-      for (int k = 0; k < K; ++k) {
-        const int fk = z0 + W * k;
-        if (!act[k] || (fk != 0 && fk != nf - 1)) continue;
-        static_for<Q>([&](auto I) {
-          constexpr int cf = D::d == 3 ? D::C[I][2] : D::C[I][1];
-          if constexpr (cf != 0) {
-            if ((cf > 0 && fk == nf - 1) || (cf < 0 && fk == 0)) {
-              constexpr int cx = D::C[I][0], cy = D::C[I][1];
-              bool inside = x + cx >= 0 && x + cx < g.nx;
-              if constexpr (D::d == 3) inside = inside && y + cy >= 0 && y + cy < g.ny;
-              if (inside) ghost_store(I, k, n0 + W * k - uint32_t(cf * nf));
+        const int x = D::d == 3 ? int(blockIdx.z) : sl[k], y = D::d == 3 ? sl[k] : fz[k], z = D::d == 3 ? fz[k] : 0;
+        const bool slowFace = ((g.pmask & 1) && (x == 0 || x == g.nx - 1)) ||
+                              (D::d == 3 && (g.pmask & 2) && (y == 0 || y == g.ny - 1));
+        if (slowFace) {
+          static_for<Q>([&](auto I) {
+            constexpr int cx = D::C[I][0], cy = D::C[I][1], cz = D::C[I][2];
+            int tx = x + cx, ty = y + cy, tz = z + cz;
+            bool crossed = false, lost = false;
+            if (tx < 0 || tx >= g.nx) { if (g.pmask & 1) { tx = tx < 0 ? tx + g.nx : tx - g.nx; crossed = true; } else lost = true; }
+            if (ty < 0 || ty >= g.ny) { if (g.pmask & 2) { ty = ty < 0 ? ty + g.ny : ty - g.ny; crossed = true; } else lost = true; }
+            if constexpr (D::d == 3) {
+              if (tz < 0 || tz >= g.nz) { if (g.pmask & 4) { tz = tz < 0 ? tz + g.nz : tz - g.nz; crossed = true; } else lost = true; }
             }
-          }
-        });
+            if (crossed && !lost) {
+              const int64_t gn = int64_t(tx - cx + 1) * g.sx + int64_t(ty - cy + 1) * g.sy + (tz - cz + g.pz);
+              ghost_store(I, k, uint32_t(gn));
+            }
+          });
+        } else if ((g.pmask & (D::d == 3 ? 4 : 2)) && (fz[k] == 0 || fz[k] == nf - 1)) {
+          static_for<Q>([&](auto I) {
+            constexpr int cf = D::d == 3 ? D::C[I][2] : D::C[I][1];
+            if constexpr (cf != 0) {
+              if ((cf > 0 && fz[k] == nf - 1) || (cf < 0 && fz[k] == 0)) {
+                constexpr int cx = D::C[I][0], cy = D::C[I][1];
+                bool in = x + cx >= 0 && x + cx < g.nx;
+                if constexpr (D::d == 3) in = in && y + cy >= 0 && y + cy < g.ny;
+                if (in) ghost_store(I, k, n0 + W * k - uint32_t(cf * nf));
+              }
+            }
+          });
+        }
       }
     }
     // halfway bounce-back (BouzidiPostProcessor with q = 1/2, boundary/setBouzidiBoundary.h:48-77,
@@ -1367,7 +1414,7 @@ __global__ void __launch_bounds__(256) k_periodic_halo(S* __restrict__ pop, Geom
 // ---- halfway bounce-back links (PostStream) ---------------------------------------------
 // f_opp(k)(x_b) = f_k(x_b + c_k) - delta, delta = 2 (c_k . u_w) t_k / c_s^2.
 template <int Q, typename S>
-__global__ void __launch_bounds__(256) k_bouzidi(S* __restrict__ pop, Geometry g, Shifts<Q> sh,
+__global__ void __launch_bounds__(256) k_bouzidi(S* pop, Geometry g, Shifts<Q> sh,
                                                  const uint32_t* __restrict__ cell,
                                                  const uint8_t* __restrict__ dir,
                                                  const typename Storage<S>::R* __restrict__ delta,
@@ -1375,9 +1422,11 @@ __global__ void __launch_bounds__(256) k_bouzidi(S* __restrict__ pop, Geometry g
   using R = typename Storage<S>::R;
   using D = Desc<Q>;
   const int64_t l = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  chain_next();
+  const int64_t xb = l < nLinks ? cell[l] : 0;
+  const int k = l < nLinks ? dir[l] : 0;
+  chain_wait();
   if (l >= nLinks) return;
-  const int64_t xb = cell[l];
-  const int k = dir[l];
   int64_t off = 0;
   int kopp = 0;
   static_for<Q>([&](auto I) {
@@ -1555,11 +1604,13 @@ __device__ __forceinline__ void bulk_velocity(const R (&f)[Q], const R (&halfF)[
   });
 }
 
+// (32-bit: a lattice has fewer than 2^32 padded cells)
 __device__ __forceinline__ void fd_decode(const Geometry& g, int64_t n, int& x, int& y, int& z) {
-  x = int(n / g.sx) - 1;
-  const int64_t r = n - int64_t(x + 1) * g.sx;
-  y = int(r / g.sy) - 1;
-  z = int(r - int64_t(y + 1) * g.sy) - int(g.pz);
+  const uint32_t sx = uint32_t(g.sx), sy = uint32_t(g.sy), px = uint32_t(n) / sx;
+  const uint32_t r = uint32_t(n) - px * sx, py = r / sy;
+  x = int(px) - 1;
+  y = int(py) - 1;
+  z = int(r - py * sy) - int(g.pz);
 }
 
 // Pi of a flat local boundary cell: RegularizedBoundaryStress (BoundaryHelpers::computeStress,
@@ -1716,7 +1767,7 @@ __device__ __forceinline__ R rlb_relax(R (&f)[Q], FdMeta m, R rho, const R (&u)[
 // on a periodic face also refreshes the ghost slots of its leaving populations (the bulk
 // kernel wrote them before this collision).  Statistics partials go after the bulk kernel's.
 template <int Q, typename S>
-__global__ void __launch_bounds__(256) k_fd_collide(S* __restrict__ pop, Geometry g, Shifts<Q> sh, double omega,
+__global__ void __launch_bounds__(256) k_fd_collide(S* pop, Geometry g, Shifts<Q> sh, double omega,
                                                     int64_t nFd, const uint32_t* __restrict__ fdCell,
                                                     const uint16_t* __restrict__ fdMeta,
                                                     const double* __restrict__ fdValue, double* __restrict__ statPart) {
@@ -1724,9 +1775,11 @@ __global__ void __launch_bounds__(256) k_fd_collide(S* __restrict__ pop, Geometr
   using D = Desc<Q>;
   const int64_t b = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   double aR = 0.0, aU = 0.0, aC = 0.0;
+  chain_next();
+  const int64_t n = b < nFd ? fdCell[b] : 0;
+  const FdMeta m(b < nFd ? fdMeta[b] : uint16_t(0));
+  chain_wait();
   if (b < nFd) {
-    const int64_t n = fdCell[b];
-    const FdMeta m(fdMeta[b]);
     R f[Q];
     static_for<Q>([&](auto I) { f[I] = Storage<S>::load(pop + I * g.stride + wrap_add(n, sh.s[I], g.n)); });
     R rho, u[3];
@@ -1781,13 +1834,15 @@ __global__ void __launch_bounds__(256) k_fd_collide(S* __restrict__ pop, Geometr
 // the ghost slots of a cell on a periodic face refreshed as k_fd_collide does; value[4 b ...] =
 // {rho, u}.  Statistics partials go after the boundary kernel's.
 template <int Q, typename S>
-__global__ void __launch_bounds__(256) k_bbv_collide(S* __restrict__ pop, Geometry g, Shifts<Q> sh, int64_t nB,
+__global__ void __launch_bounds__(256) k_bbv_collide(S* pop, Geometry g, Shifts<Q> sh, int64_t nB,
                                                      const uint32_t* __restrict__ bCell,
                                                      const double* __restrict__ bValue, double* __restrict__ statPart) {
   using R = typename Storage<S>::R;
   using D = Desc<Q>;
   const int64_t b = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   double aR = 0.0, aU = 0.0, aC = 0.0;
+  chain_next();
+  chain_wait();
   if (b < nB) {
     const int64_t n = bCell[b];
     R f[Q];
@@ -1835,20 +1890,23 @@ __global__ void __launch_bounds__(256) k_bbv_collide(S* __restrict__ pop, Geomet
 // copy of the cell, which carries bulk dynamics), from the populations before any cell is
 // rewritten.  fdMom[7 b ...] = {u, u_bulk, rho}.
 template <int Q, typename S>
-__global__ void __launch_bounds__(256) k_fd_momenta(const S* __restrict__ pop, Geometry g, Shifts<Q> sh, int64_t nFd,
+__global__ void __launch_bounds__(256) k_fd_momenta(const S* pop, Geometry g, Shifts<Q> sh, int64_t nFd,
                                                     const uint32_t* __restrict__ fdCell,
                                                     const uint16_t* __restrict__ fdMeta,
                                                     const double* __restrict__ fdValue, double hfx, double hfy,
-                                                    double hfz, double* __restrict__ fdMom) {
+                                                    double hfz, double* fdMom) {
   using R = typename Storage<S>::R;
   const int64_t b = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  chain_next();
+  const int64_t n = b < nFd ? fdCell[b] : 0;
+  const FdMeta m(b < nFd ? fdMeta[b] : uint16_t(0));
+  chain_wait();
   if (b >= nFd) return;
-  const int64_t n = fdCell[b];
   R f[Q];
   static_for<Q>([&](auto I) { f[I] = Storage<S>::load(pop + I * g.stride + wrap_add(n, sh.s[I], g.n)); });
   R rho, u[3], ub[3];
   const R halfF[3] = {R(hfx), R(hfy), R(hfz)};
-  fd_momenta<Q, R>(f, FdMeta(fdMeta[b]), fdValue + 4 * b, rho, u);
+  fd_momenta<Q, R>(f, m, fdValue + 4 * b, rho, u);
   bulk_velocity<Q, R>(f, halfF, ub);
   double* out = fdMom + 7 * b;
   for (int a = 0; a < 3; ++a) {
@@ -1878,12 +1936,12 @@ __global__ void __launch_bounds__(256) k_fd_momenta(const S* __restrict__ pop, G
 // populations, i.e. those the priority-0 processors left, as the reference's corner processor
 // reads them.
 template <int Q, typename S>
-__global__ void __launch_bounds__(256) k_fd_regularize(S* __restrict__ pop, Geometry g, Shifts<Q> sh, double omega,
+__global__ void __launch_bounds__(256) k_fd_regularize(S* pop, Geometry g, Shifts<Q> sh, double omega,
                                                        int64_t nFd, const uint32_t* __restrict__ fdCell,
                                                        const uint16_t* __restrict__ fdMeta,
                                                        const double* __restrict__ fdValue,
                                                        const uint8_t* __restrict__ cellDyn, double hfx, double hfy,
-                                                       double hfz, const double* __restrict__ fdMom, int corners,
+                                                       double hfz, const double* fdMom, int corners,
                                                        int64_t nBbv, const uint32_t* __restrict__ bbvCell,
                                                        const double* __restrict__ bbvValue,
                                                        const int32_t* __restrict__ bIdx) {
@@ -1898,10 +1956,13 @@ __global__ void __launch_bounds__(256) k_fd_regularize(S* __restrict__ pop, Geom
   // the other this took the pass from 22 to 19 us a launch on a 128 x 64 x 64 channel; a warp per
   // cell, every lane repeating the cell's arithmetic, was slower at 26 us.)
   const int64_t b = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (b >= nFd) return;
-  const FdMeta m(fdMeta[b]);
-  if (m.local) return;  // local boundaries have no post-processor
-  if ((m.type == FD_CORNER_VELOCITY) != (corners != 0)) return;
+  chain_next();
+  const FdMeta m(b < nFd ? fdMeta[b] : uint16_t(0));
+  // local boundaries have no post-processor
+  if (b >= nFd || m.local || (m.type == FD_CORNER_VELOCITY) != (corners != 0)) {
+    chain_wait();
+    return;
+  }
   const int64_t n = fdCell[b];
   int pos[3];
   fd_decode(g, n, pos[0], pos[1], pos[2]);
@@ -1975,6 +2036,7 @@ __global__ void __launch_bounds__(256) k_fd_regularize(S* __restrict__ pop, Geom
   uint8_t kind[NS];
 #pragma unroll
   for (int s = 0; s < NS; ++s) kind[s] = (use[s] && bi[s] < 0 && cellDyn) ? cellDyn[nn[s]] : uint8_t(1);
+  chain_wait();  // the neighbours' places and kinds above are set-up data
   R nv[6][3], nr[6];
   bool pend[NS];  // the value comes from the cell's populations
 #pragma unroll
@@ -2311,8 +2373,33 @@ struct LaunchArgs {
 // thread K cells a warp apart (k_collide_stream_groups).
 inline int k_cells_threads(int nf, int K) { return K == 1 ? nf : (nf + 32 * K - 1) / (32 * K) * 32; }
 
-// Blocks of 256 threads the boundary-cell collision adds to a step's statistics partials.
-inline int64_t fd_blocks(int64_t nFd) { return (nFd + 255) / 256; }
+// Grid of the K-cells step kernel.  Its threads go by rows of the core, or flat through the padded
+// cells of a plane where that leaves fewer lanes idle: rows waste what the row lacks to a multiple
+// of 32 K cells (nz = 97 at K = 1: 24 %), flat the two padding cells of each row.  Where rows fill
+// their lanes they are kept: no division per cell, and no padding lanes.  Variant 5 prefetches rows.
+struct GroupsShape {
+  unsigned x, y, z;
+  bool flat;
+};
+inline GroupsShape groups_shape(int d, const Geometry& g, int kernel, int K, int bx, int by) {
+  const int64_t nf = d == 3 ? g.nz : g.ny, rows = d == 3 ? g.ny : g.nx, planes = d == 3 ? g.nx : 1;
+  const int64_t lanes = k_cells_threads(int(nf), K);
+  const int64_t rowLanes = ((lanes + bx - 1) / bx * bx) * ((rows + by - 1) / by * by) * K;
+  const int64_t cells = (rows - 1) * (d == 3 ? g.sy : g.sx) + nf, per = int64_t(bx) * by * K;
+  const int64_t flatBlocks = (cells + per - 1) / per;
+  GroupsShape s;
+  s.flat = kernel == 2 && flatBlocks * per * 21 < rowLanes * 20;
+  s.x = unsigned(s.flat ? flatBlocks : (lanes + bx - 1) / bx);
+  s.y = unsigned(s.flat ? 1 : (rows + by - 1) / by);
+  s.z = unsigned(planes);
+  return s;
+}
+
+// Boundary cells a block of their kernels takes: one thread's serial work per cell, so small blocks,
+// which spread a boundary over more SMs.
+constexpr int kFdThreads = 64;
+// Blocks the boundary-cell collision adds to a step's statistics partials.
+inline int64_t fd_blocks(int64_t nFd) { return (nFd + kFdThreads - 1) / kFdThreads; }
 
 // How far ahead in launch order the step kernel prefetches into L2: one wave of resident blocks
 // (the block that takes over a finishing block's SM).  `cache` belongs to one kernel: per device,
@@ -2510,15 +2597,15 @@ cudaError_t launch_step_dyn(const LaunchArgs& a, cudaStream_t stream) {
       cols.s[i] = a.doubled ? 0u : uint32_t(a.shift[i]);
     }
     const int K = a.cellsPerThread;
-    const int nf = Desc<Q>::d == 3 ? g.nz : g.ny;
-    const int groups = k_cells_threads(nf, K);
-    dim3 block(a.blockX, a.blockY, 1);
-    dim3 grid;
-    if (Desc<Q>::d == 3) grid = dim3((groups + a.blockX - 1) / a.blockX, (g.ny + a.blockY - 1) / a.blockY, g.nx);
-    else grid = dim3((groups + a.blockX - 1) / a.blockX, (g.nx + a.blockY - 1) / a.blockY, 1);
+    const GroupsShape shape = groups_shape(Desc<Q>::d, g, a.kernel, K, a.blockX, a.blockY);
+    const dim3 block(a.blockX, a.blockY, 1), grid(shape.x, shape.y, shape.z);
+    FlatDiv dv;
+    FlatDiv::make(uint32_t(g.sx), dv.mx, dv.lx);
+    FlatDiv::make(uint32_t(g.sy), dv.my, dv.ly);
     nblocks = int64_t(grid.x) * grid.y * grid.z;
     if (a.stats && nblocks > a.statCapacity) return cudaErrorInvalidValue;
     double* part = a.stats ? a.statPart : nullptr;
+    cudaError_t chained = cudaSuccess;
     auto go = [&](auto kk, auto doubled, auto mapped) {
       auto kern =
           k_collide_stream_groups<Q, S, DYN, decltype(kk)::value, decltype(doubled)::value, decltype(mapped)::value>;
@@ -2526,8 +2613,8 @@ cudaError_t launch_step_dyn(const LaunchArgs& a, cudaStream_t stream) {
       int ahead = 0;
       if constexpr (decltype(doubled)::value)
         if (a.kernel == 5) ahead = l2_ahead_blocks(kern, int(block.x * block.y), aheadCache);
-      kern<<<grid, block, 0, stream>>>(cols, g, p, a.cellDyn, a.linkMask, static_cast<const R*>(a.wallDelta), part,
-                                       ahead);
+      chained = launch_chained(kern, grid, block, stream, cols, g, p, a.cellDyn, a.linkMask,
+                               static_cast<const R*>(a.wallDelta), part, ahead, shape.flat ? 1 : 0, dv);
     };
     auto go_k = [&](auto kk) {
       if (a.doubled) {
@@ -2551,6 +2638,7 @@ cudaError_t launch_step_dyn(const LaunchArgs& a, cudaStream_t stream) {
       return cudaErrorInvalidValue;
     default: return cudaErrorInvalidValue;
     }
+    if (chained != cudaSuccess) return chained;
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
@@ -2558,23 +2646,21 @@ cudaError_t launch_step_dyn(const LaunchArgs& a, cudaStream_t stream) {
   if (a.nFd > 0) {
     fdb = fd_blocks(a.nFd);
     if (a.stats && nblocks + fdb > a.statCapacity) return cudaErrorInvalidValue;
-    k_fd_collide<Q, S><<<unsigned(fdb), 256, 0, stream>>>(pop, g, sh, a.omega, a.nFd, a.fdCell, a.fdMeta, a.fdValue,
-                                                          a.stats ? a.statPart + 4 * nblocks : nullptr);
-    e = cudaGetLastError();
+    e = launch_chained(k_fd_collide<Q, S>, dim3(unsigned(fdb)), dim3(kFdThreads), stream, pop, g, sh, a.omega, a.nFd,
+                       a.fdCell, a.fdMeta, a.fdValue, a.stats ? a.statPart + 4 * nblocks : nullptr);
     if (e != cudaSuccess) return e;
   }
   int64_t bbb = 0;
   if (a.nBbv > 0) {
     bbb = fd_blocks(a.nBbv);
     if (a.stats && nblocks + fdb + bbb > a.statCapacity) return cudaErrorInvalidValue;
-    k_bbv_collide<Q, S><<<unsigned(bbb), 256, 0, stream>>>(pop, g, sh, a.nBbv, a.bbvCell, a.bbvValue,
-                                                           a.stats ? a.statPart + 4 * (nblocks + fdb) : nullptr);
-    e = cudaGetLastError();
+    e = launch_chained(k_bbv_collide<Q, S>, dim3(unsigned(bbb)), dim3(kFdThreads), stream, pop, g, sh, a.nBbv, a.bbvCell,
+                       a.bbvValue, a.stats ? a.statPart + 4 * (nblocks + fdb) : nullptr);
     if (e != cudaSuccess) return e;
   }
   if (!a.stats) return cudaSuccess;
-  k_stats_finalize<<<1, kFinalizeThreads, 0, stream>>>(a.statPart, nblocks + fdb + bbb, a.stats);
-  return cudaGetLastError();
+  return launch_chained(k_stats_finalize, dim3(1), dim3(kFinalizeThreads), stream, a.statPart, nblocks + fdb + bbb,
+                        a.stats);
 }
 // Post-stream regularisation of the boundary cells: momenta, then flat faces and edges, then
 // corners (see k_fd_regularize).
@@ -2587,15 +2673,13 @@ cudaError_t launch_fd_boundary(const LaunchArgs& a, cudaStream_t stream) {
   // forced bulk neighbours report j / rho + F / 2 (ForcedMomentum)
   const bool forced = a.dynamics == DYN_FORCED_BGK || a.dynamics == DYN_FORCED_SMAGORINSKY;
   const double hf[3] = {forced ? 0.5 * a.force[0] : 0.0, forced ? 0.5 * a.force[1] : 0.0, forced ? 0.5 * a.force[2] : 0.0};
-  k_fd_momenta<Q, S><<<blocks, 256, 0, stream>>>(pop, a.g, sh, a.nFd, a.fdCell, a.fdMeta, a.fdValue, hf[0], hf[1],
-                                                 hf[2], a.fdMom);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_chained(k_fd_momenta<Q, S>, dim3(blocks), dim3(kFdThreads), stream, pop, a.g, sh, a.nFd, a.fdCell,
+                                 a.fdMeta, a.fdValue, hf[0], hf[1], hf[2], a.fdMom);
   if (e != cudaSuccess) return e;
   for (int corners = 0; corners < (a.nFdCorners > 0 ? 2 : 1); ++corners) {
-    k_fd_regularize<Q, S><<<blocks, 256, 0, stream>>>(pop, a.g, sh, a.omega, a.nFd, a.fdCell, a.fdMeta, a.fdValue,
-                                                      a.cellDyn, hf[0], hf[1], hf[2], a.fdMom, corners, a.nBbv,
-                                                      a.bbvCell, a.bbvValue, a.bIdx);
-    e = cudaGetLastError();
+    e = launch_chained(k_fd_regularize<Q, S>, dim3(blocks), dim3(kFdThreads), stream, pop, a.g, sh, a.omega, a.nFd,
+                       a.fdCell, a.fdMeta, a.fdValue, a.cellDyn, hf[0], hf[1], hf[2], a.fdMom, corners, a.nBbv,
+                       a.bbvCell, a.bbvValue, a.bIdx);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
@@ -2636,9 +2720,8 @@ cudaError_t launch_bouzidi(const LaunchArgs& a, const uint32_t* cell, const uint
   using R = typename Storage<S>::R;
   if (nLinks <= 0) return cudaSuccess;
   const int64_t blocks = (nLinks + 255) / 256;
-  k_bouzidi<Q, S><<<unsigned(blocks), 256, 0, stream>>>(static_cast<S*>(a.pop), a.g, shifts_of<Q>(a), cell, dir,
-                                                        static_cast<const R*>(delta), nLinks);
-  return cudaGetLastError();
+  return launch_chained(k_bouzidi<Q, S>, dim3(unsigned(blocks)), dim3(256), stream, static_cast<S*>(a.pop), a.g,
+                        shifts_of<Q>(a), cell, dir, static_cast<const R*>(delta), nLinks);
 }
 template <int Q, typename S>
 cudaError_t launch_transfer(const LaunchArgs& a, int i, const void* stage, int hostType, bool toColumns,

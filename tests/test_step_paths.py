@@ -1,5 +1,6 @@
-"""Paths that a step can take give the same bits: the packed two-cell collision against the scalar
-one, for every dynamics, on lattices whose cell pairs mix bulk cells with solid and bounce-back ones."""
+"""Paths that a step can take give the same bits: the packed two-cell collision and the flat mapping of
+threads to cells against one thread per cell by rows, for every dynamics, on lattices whose cell pairs
+mix bulk cells with solid and bounce-back ones; fused moving walls against the link kernel."""
 import numpy as np
 import pytest
 
@@ -46,9 +47,9 @@ def populations(lat):
 def test_packed_pairs_match_single_cells(dynamics, q, core, storage):
     for kw in ({}, {"solid": 0.3}, {"bounce": 0.1, "solid": 0.1}):
         ref = None
-        for cells in (1, 2):
+        for variant, cells in ((1, 1), (2, 1), (2, 2)):
             lat = lattice(q, core, (1, 1, 1 if q != 9 else 0), storage, dynamics, **kw)
-            lat.set_launch_config(2, 32, 4, cells)
+            lat.set_launch_config(variant, 32, 4, cells)
             for _ in range(6):
                 lat.collide_and_stream(1)
             f = populations(lat)
@@ -57,6 +58,25 @@ def test_packed_pairs_match_single_cells(dynamics, q, core, storage):
                 ref = f
             else:
                 assert np.array_equal(ref, f)
+
+
+@pytest.mark.parametrize("storage", ["f64", "f32"])
+@pytest.mark.parametrize("q,core", [(19, (3, 4, 1)), (19, (2, 3, 32)), (19, (5, 7, 33)), (19, (4, 9, 161)),
+                                    (27, (3, 5, 65)), (9, (5, 31)), (9, (1, 97)), (9, (40, 129))])
+def test_ragged_rows_match_one_thread_per_cell(q, core, storage):
+    """Rows that fill their lanes and rows that do not (the step then runs flat through the padded
+    cells), periodic on all axes and on some."""
+    for periodic in ((1, 1, 1), (0, 1, 0), (1, 0, 1)):
+        periodic = periodic if q != 9 else (periodic[0], periodic[1], 0)
+        ref = None
+        for variant, block in ((1, (32, 8)), (2, (32, 4)), (2, (128, 1)), (2, (256, 1))):
+            lat = lattice(q, core, periodic, storage, "bgk")
+            lat.set_launch_config(variant, *block, 1)
+            for _ in range(5):
+                lat.collide_and_stream(1)
+            f = populations(lat)
+            ref = f if ref is None else ref
+            assert np.array_equal(ref, f)
 
 
 @pytest.mark.parametrize("storage", ["f64", "f32", "f16dev"])
