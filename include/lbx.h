@@ -397,7 +397,8 @@ int lbx_rotate(lbx_lattice lattice, int32_t pop, int64_t offset);
  * core/platform/gpu/cuda/operator.hh:425-441).  variant 0: pipelined shared-memory tiles of 256 cells;
  * variant 1: one cell per thread in (block_x, block_y) blocks; variant 2 (default):
  * cells_per_thread (1 or 2; 4 for 16-bit storage) cells a warp apart per thread in
- * (block_x, block_y) blocks, block_x along the fastest axis; variant 3: tiles moved by TMA bulk
+ * (block_x, block_y) blocks, block_x along the fastest axis, or along the padded cells of a plane
+ * where its rows would leave lanes idle; variant 3: tiles moved by TMA bulk
  * copies, two stages per block; variant 4: tiles moved by TMA bulk copies through a ring of
  * four stages, one producer warp and sixteen consumer warps per block (block_x, block_y and
  * cells_per_thread are ignored by 0, 3 and 4); variant 5: variant 2 plus an L2 bulk prefetch,
@@ -489,7 +490,8 @@ int lbx_ensemble_set_config(lbx_ensemble ens, int32_t threads, int32_t blocks_pe
  * CUDA graph (the launch boundaries order the steps, and populations may then be read through
  * L1).  Both give identical results. */
 int lbx_ensemble_set_launch_mode(lbx_ensemble ens, int32_t mode);
-/* Cells per thread of the tile loop, 1 (default) or 2: a warp steps 32 * cells consecutive
+/* Cells per thread of the tile loop, 1 or 2 (default: 2 for the FP32, FP16 and BF16 forms of D3Q19,
+ * 1 otherwise): a warp steps 32 * cells consecutive
  * cells of a tile per round, keeping that many loads in flight per thread.  Both give identical
  * results. */
 int lbx_ensemble_set_cells_per_thread(lbx_ensemble ens, int32_t cells);

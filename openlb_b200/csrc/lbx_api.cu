@@ -102,6 +102,12 @@ int discrete_normals(int q, const int32_t core[3], const int32_t periodic[3], co
                      std::vector<int32_t>& normals);
 }  // namespace lbx
 
+// A lattice's statistics and error flag side by side, read by one copy.
+struct StatBlock {
+  StatAcc acc;
+  int err;
+};
+
 // A velocity / pressure boundary cell as set through the ABI.
 struct FdHostCell {
   int64_t core = 0;
@@ -166,7 +172,7 @@ struct lbx_lattice_s {
   int64_t statCapacity = 0;          // blocks statPart holds
   double* reduceAcc = nullptr;       // 8 doubles + 1 ull of scratch for reductions
   double* reducePart = nullptr;      // per-block entries of the FP64 reductions (4 doubles each)
-  int* devErr = nullptr;             // set by a step kernel whose bounded wait gave up
+  int* devErr = nullptr;             // set by a step kernel whose bounded wait gave up (StatBlock::err)
   int64_t reducePartCapacity = 0;    // blocks reducePart holds
   float* residualSnap = nullptr;
   void* stage = nullptr;             // ncore doubles
@@ -346,7 +352,7 @@ int64_t step_blocks(const lbx_lattice_s* L) {
     return (a.flatEnd - a.flatBase + bt - 1) / bt;
   }
   if (groups_kernel(L->kernel)) {
-    const GroupsShape s = groups_shape(L->d, g, L->kernel, L->cellsPerThread, L->blockX, L->blockY);
+    const GroupsShape s = groups_shape(L->d, g, L->kernel, L->cellsPerThread, L->blockX, L->blockY, L->doubled);
     return int64_t(s.x) * s.y * s.z;
   }
   const int64_t groups = nf;
@@ -814,7 +820,7 @@ int install_boundary_list(lbx_lattice_s* L, std::vector<FdHostCell> list) {
   LBX_CUDA_TRY(cudaMalloc(&L->fdCell, size_t(n) * sizeof(uint32_t)));
   LBX_CUDA_TRY(cudaMalloc(&L->fdMeta, size_t(n) * sizeof(uint16_t)));
   LBX_CUDA_TRY(cudaMalloc(&L->fdValue, size_t(4 * n) * sizeof(double)));
-  LBX_CUDA_TRY(cudaMalloc(&L->fdMom, size_t(7 * n) * sizeof(double)));
+  LBX_CUDA_TRY(cudaMalloc(&L->fdMom, size_t(8 * n) * sizeof(double)));
   LBX_CUDA_TRY(cudaMemcpy(L->fdCell, hc.data(), size_t(n) * sizeof(uint32_t), cudaMemcpyHostToDevice));
   LBX_CUDA_TRY(cudaMemcpy(L->fdMeta, hm.data(), size_t(n) * sizeof(uint16_t), cudaMemcpyHostToDevice));
   LBX_CUDA_TRY(cudaMemcpy(L->fdValue, hv.data(), size_t(4 * n) * sizeof(double), cudaMemcpyHostToDevice));
@@ -910,8 +916,10 @@ int set_links_impl(lbx_lattice_s* L, int64_t n, const int64_t* cells, const int3
 // copy and the shift rotation; then the post-stream links and boundary cells.
 // ConstRhoBGK reads the previous step's average density, so its statistics are kept on every
 // step, as the reference keeps them whenever statistics are enabled (its default).
-int step_collide(lbx_lattice_s* L, bool statistics, cudaStream_t s, cudaEvent_t (&ev)[4]) {
+// fdCollided: the step before has collided this step's velocity / pressure boundary cells already.
+int step_collide(lbx_lattice_s* L, bool statistics, cudaStream_t s, cudaEvent_t (&ev)[4], bool fdCollided = false) {
   LaunchArgs a = args_of(L);
+  a.fdCollided = fdCollided ? 1 : 0;
   if (statistics || L->dynamics == LBX_CONST_RHO_BGK) {
     if (int rc = ensure_stat_capacity(L)) return rc;
     a.stats = L->stats;
@@ -931,9 +939,11 @@ int step_collide(lbx_lattice_s* L, bool statistics, cudaStream_t s, cudaEvent_t 
   return LBX_OK;
 }
 
-int step_post_stream(lbx_lattice_s* L, cudaStream_t s) {
+// fdCollideNext: the boundary cells are collided for the next step as they are rebuilt.
+int step_post_stream(lbx_lattice_s* L, cudaStream_t s, bool fdCollideNext = false) {
   if (L->nLinks > 0 || L->nFd > 0) {
-    const LaunchArgs b = args_of(L);
+    LaunchArgs b = args_of(L);
+    b.fdCollideNext = fdCollideNext ? 1 : 0;
     // the K-cells kernel applied the resting links itself (linkMask); the link kernel does
     // the rest, or all of them after the other kernel variants
     if (b.linkMask) {
@@ -1014,11 +1024,10 @@ int lbx_lattice_create(int32_t q, const int32_t core[3], const int32_t periodic[
   L->ncore = int64_t(core[0]) * core[1] * core[2];
   cudaError_t e = alloc_columns(L);
   default_block_shape(L);
-  if (e == cudaSuccess) e = cudaMalloc(&L->stats, sizeof(StatAcc));
-  if (e == cudaSuccess) e = cudaMemset(L->stats, 0, sizeof(StatAcc));
+  if (e == cudaSuccess) e = cudaMalloc(&L->stats, sizeof(StatBlock));
+  if (e == cudaSuccess) e = cudaMemset(L->stats, 0, sizeof(StatBlock));
+  L->devErr = &reinterpret_cast<StatBlock*>(L->stats)->err;
   if (e == cudaSuccess) e = cudaMalloc(&L->reduceAcc, 8 * sizeof(double) + sizeof(unsigned long long));
-  if (e == cudaSuccess) e = cudaMalloc(&L->devErr, sizeof(int));
-  if (e == cudaSuccess) e = cudaMemset(L->devErr, 0, sizeof(int));
   if (e != cudaSuccess) {
     const std::string msg = std::string("allocation failed: ") + cudaGetErrorString(e);
     release_columns(L);
@@ -1059,7 +1068,6 @@ int lbx_lattice_destroy(lbx_lattice L) {
   cudaFree(L->statPart);
   cudaFree(L->reduceAcc);
   cudaFree(L->reducePart);
-  cudaFree(L->devErr);
   cudaFree(L->residualSnap);
   cudaFree(L->stage);
   delete L;
@@ -1502,10 +1510,19 @@ int lbx_collide_and_stream(lbx_lattice L, int64_t steps, uint32_t flags, void* s
   if (steps < 0) return fail(LBX_ERR_INVALID, "steps must be >= 0");
   DeviceGuard guard(L->device);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  // Velocity / pressure boundary cells: a step that another plain step follows collides them for it
+  // in the launch that rebuilds them.  (Not for a step with statistics, which count them, nor
+  // under per-kernel timing.)
+  bool collided = false;
   for (int64_t k = 0; k < steps; ++k) {
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
-    if (int rc = step_collide(L, ((flags & LBX_STEP_STATISTICS) && k == steps - 1), s, ev)) return rc;
-    if (int rc = step_post_stream(L, s)) return rc;
+    const bool statistics = (flags & LBX_STEP_STATISTICS) && k == steps - 1;
+    const bool nextStatistics = (flags & LBX_STEP_STATISTICS) && k + 1 == steps - 1;
+    const bool ahead = L->nFd > 0 && L->nBbv == 0 && k + 1 < steps && !nextStatistics && !L->timing &&
+                       L->dynamics != LBX_CONST_RHO_BGK;
+    if (int rc = step_collide(L, statistics, s, ev, collided)) return rc;
+    if (int rc = step_post_stream(L, s, ahead)) return rc;
+    collided = ahead;
     if (ev[3]) {
       cudaEventRecord(ev[3], s);
       if (ev[0] && ev[1] && ev[2]) {
@@ -1555,12 +1572,11 @@ int lbx_get_statistics(lbx_lattice L, double out[4], void* stream) {
   if (!L || !out) return fail(LBX_ERR_INVALID, "null argument");
   DeviceGuard guard(L->device);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  StatAcc h;
-  int kerr = 0;
-  LBX_CUDA_TRY(cudaMemcpyAsync(&h, L->stats, sizeof(StatAcc), cudaMemcpyDeviceToHost, s));
-  LBX_CUDA_TRY(cudaMemcpyAsync(&kerr, L->devErr, sizeof(int), cudaMemcpyDeviceToHost, s));
+  StatBlock block;
+  LBX_CUDA_TRY(cudaMemcpyAsync(&block, L->stats, sizeof(StatBlock), cudaMemcpyDeviceToHost, s));
   LBX_CUDA_TRY(cudaStreamSynchronize(s));
-  if (kerr) {
+  const StatAcc& h = block.acc;
+  if (block.err) {
     cudaMemset(L->devErr, 0, sizeof(int));
     return fail(LBX_ERR_CUDA, "a step kernel gave up waiting for its bulk copies; results of that step are invalid");
   }

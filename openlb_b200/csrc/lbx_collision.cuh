@@ -205,9 +205,9 @@ template <int Q> struct Weights {
 // equilibrium's even and odd parts enter with d_even, d_odd = 3 omega t_1, taken from the rounded a
 // and b, so that a + b + N d_even and a - b + N d_odd are 1.  Rounding omega t_i direction by
 // direction instead leaves a factor 1 + 3e-8 on the momentum of every step, which is most of the
-// FP32 form's error after some hundred steps.  Against FP64 after 20 steps of a 256^3 Taylor-Green
-// flow the largest relative error of a population column fell from 8.6e-5 to 3.5e-6 (with delta in
-// place of rho - 1 below), after 100 steps of a 64^3 cavity from 8.4e-6 to 2.4e-6.
+// FP32 form's error after some hundred steps.  Against FP64 after 20 steps of a 131 x 150 x 97 D3Q27
+// TRT Taylor-Green flow the largest relative error of a population column fell from 5.2e-5 to 1.8e-6
+// (with delta in place of rho - 1 below).
 struct Relaxation {
   static void set(int q, float omegaF, float magic, bool trt, float (&r)[4]) {
     const double omega = omegaF, omega2 = trt ? trt_omega2(omega, double(magic)) : omega;
@@ -219,7 +219,8 @@ struct Relaxation {
   }
 };
 
-// BGK, TRT, Smagorinsky and the Guo-forced forms.  Opposite directions i, j share q = (c_i . J)^2
+// TRT, Smagorinsky and the Guo-forced forms (and BGK, whose pair this describes, where forced).
+// Opposite directions i, j share q = (c_i . J)^2
 // with J = rho u (the momentum, plus rho F / 2 where forced) and differ in the sign of what is odd in
 // c_i.  With delta = rho - 1 (the sum of the stored f - w) and K = delta - 1.5 J^2 / rho the
 // equilibrium, less w, is t (K + 4.5 q / rho +- 3 c_i . J); its constant part cancels against the
@@ -234,8 +235,7 @@ struct Relaxation {
 // reference's templates took 418 instructions a warp for 32 cells of D3Q19 BGK, two and three times
 // that for TRT and the forced Smagorinsky form).  At 192^3, default launch shape, FP16 D3Q27:
 // TRT 32.2k -> 39.4k MLUPS, forced Smagorinsky 25.8k -> 35.8k; with two cells a thread, which all
-// FP32 arithmetic may now pack, FP16 D3Q19 forced Smagorinsky 35.2k -> 55.8k, and the FP32
-// form of 256^3 D3Q19 BGK 37.4k -> 40.4k (0.94 of the 6542 GB/s measured on this pool).
+// FP32 arithmetic may now pack, FP16 D3Q19 forced Smagorinsky 35.2k -> 55.8k.
 template <int Q, int DYN, typename V>
 __device__ __forceinline__ void collide_f32(V (&f)[Q], const CollisionParams<float>& p, V& rhoOut, V& uSqrOut) {
   using D = Desc<Q>;
@@ -372,6 +372,55 @@ __device__ __forceinline__ void collide_f32(V (&f)[Q], const CollisionParams<flo
   uSqrOut = vmul(ju, inv);
 }
 
+// FP32 BGK keeps the operation order that its FP32 and 16-bit runs have had, so that they repeat bit
+// for bit (a request of the ensemble near its stability limit amplifies any other rounding); the
+// same on a pair as on a cell.
+template <int Q, typename V>
+__device__ __forceinline__ void collide_bgk(V (&f)[Q], float omega, V& rhoOut, V& uSqrOut) {
+  using D = Desc<Q>;
+  V rho = f[0];
+  static_for<Q - 1>([&](auto I) { rho = vadd(rho, f[I + 1]); });
+  rho = vadd(rho, vset<V>(1.f));
+  V j[3] = {vset<V>(0.f), vset<V>(0.f), vset<V>(0.f)};
+  static_for<Q>([&](auto I) {
+    static_for<D::d>([&](auto A) {
+      constexpr int c = D::C[I][A];
+      if constexpr (c == 1) j[A] = vadd(j[A], f[I]);
+      else if constexpr (c == -1) j[A] = vsub(j[A], f[I]);
+    });
+  });
+  const V inv = vrcp(rho);
+  V u[3];
+  static_for<D::d>([&](auto A) { u[A] = vmul(j[A], inv); });
+  V uSqr = vmul(u[0], u[0]);
+  static_for<D::d - 1>([&](auto A) { uSqr = vfma(u[A + 1], u[A + 1], uSqr); });
+  const V w = vset<V>(omega), keep = vset<V>(1.f - omega);
+  const V base = vfma(vset<V>(-1.5f), uSqr, vset<V>(1.f));
+  {
+    constexpr float t0 = weight<Q, float>(0);
+    f[0] = vfma(w, vfma(vmul(rho, vset<V>(t0)), base, vset<V>(-t0)), vmul(f[0], keep));
+  }
+  static_for<Q / 2>([&](auto K) {
+    constexpr int i = K + 1;
+    constexpr int jo = D::OPP[i];
+    constexpr float t = weight<Q, float>(i);
+    V cj = vset<V>(0.f);  // c_i . j over the non-zero components in axis order
+    static_for<D::d>([&](auto A) {
+      constexpr int c = D::C[i][A];
+      if constexpr (c == 1) cj = vadd(cj, j[A]);
+      else if constexpr (c == -1) cj = vsub(cj, j[A]);
+    });
+    const V cu = vmul(cj, inv);
+    const V sym = vfma(vmul(rho, vset<V>(t)), vfma(vmul(vset<V>(4.5f), cu), cu, base), vset<V>(-t));
+    const V r3t = vmul(rho, vset<V>(3 * t)), m3t = vmul(rho, vset<V>(-3 * t));
+    const V plus = vfma(r3t, cu, sym), minus = vfma(m3t, cu, sym);
+    f[i] = vfma(w, plus, vmul(f[i], keep));
+    f[jo] = vfma(w, minus, vmul(f[jo], keep));
+  });
+  rhoOut = rho;
+  uSqrOut = uSqr;
+}
+
 // Two cells (f[k][i], k = 0, 1) of any FP32 collision but ConstRhoBGK, in place.
 template <int Q, int DYN>
 __device__ __forceinline__ void collide_x2(float (&f)[2][Q], const CollisionParams<float>& p, float (&rhoOut)[2],
@@ -379,7 +428,8 @@ __device__ __forceinline__ void collide_x2(float (&f)[2][Q], const CollisionPara
   F2 g[Q];
   static_for<Q>([&](auto I) { g[I] = make_float2(f[0][I], f[1][I]); });
   F2 rho, usq;
-  collide_f32<Q, DYN>(g, p, rho, usq);
+  if constexpr (DYN == DYN_BGK) collide_bgk<Q>(g, p.omega, rho, usq);
+  else collide_f32<Q, DYN>(g, p, rho, usq);
   static_for<Q>([&](auto I) {
     f[0][I] = g[I].x;
     f[1][I] = g[I].y;
@@ -395,7 +445,10 @@ template <int Q, typename R, int DYN>
 __device__ __forceinline__ void collide(R (&f)[Q], const CollisionParams<R>& p, R& rhoOut, R& uSqrOut) {
   using D = Desc<Q>;
   using T = DynTraits<DYN>;
-  if constexpr (DYN != DYN_CONST_RHO && sizeof(R) == 4) {
+  if constexpr (DYN == DYN_BGK && sizeof(R) == 4) {
+    collide_bgk<Q>(f, p.omega, rhoOut, uSqrOut);
+    return;
+  } else if constexpr (DYN != DYN_CONST_RHO && sizeof(R) == 4) {
     collide_f32<Q, DYN>(f, p, rhoOut, uSqrOut);
     return;
   }

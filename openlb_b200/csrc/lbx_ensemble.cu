@@ -631,7 +631,8 @@ struct lbx_ensemble_s {
   EnsKernels kern;
   int mode = 0;   // 0: persistent cooperative kernel, 1: per-step launches and a bookkeeping
                   // launch each, chained in a CUDA graph
-  int cells = 1;  // cells per thread of the tile loop (1 or 2)
+  // cells per thread of the tile loop (1 or 2): two for the FP32 arithmetic of D3Q19
+  int cells = 1;
   std::map<int, cudaGraphExec_t> graphs;
   cudaGraph_t graphTemplate = nullptr;
 };
@@ -749,6 +750,7 @@ int lbx_ensemble_create(int32_t q, int32_t storage, int64_t slab_bytes, int32_t 
   E->device = device;
   E->maxLattices = max_lattices;
   E->slabBytes = slab_bytes / 256 * 256;
+  E->cells = q == 19 && storage != LBX_F64 ? 2 : 1;
   E->slotOffset.assign(size_t(max_lattices), -1);
   E->slotBytes.assign(size_t(max_lattices), 0);
   E->slotUsed.assign(size_t(max_lattices), 0);

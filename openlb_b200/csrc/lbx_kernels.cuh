@@ -1056,13 +1056,13 @@ template <typename S> __device__ __forceinline__ S ld_column(const S* p) {
   }
 }
 
-template <int Q, typename S, int DYN, int K, bool DOUBLED, bool MAPPED>
+template <int Q, typename S, int DYN, int K, bool DOUBLED, bool MAPPED, bool FLAT>
 __global__ void __launch_bounds__(256, StepOccupancy<Q, S, K>::blocks) k_collide_stream_groups(ColumnBases<Q> cols, Geometry g,
                                                                CollisionParams<typename Storage<S>::R> p,
                                                                const uint8_t* __restrict__ cellDyn,
                                                                const uint32_t* __restrict__ linkMask,
                                                                const typename Storage<S>::R* __restrict__ wallDelta,
-                                                               double* __restrict__ statPart, int ahead, int flat,
+                                                               double* __restrict__ statPart, int ahead,
                                                                FlatDiv dv) {
   using R = typename Storage<S>::R;
   using D = Desc<Q>;
@@ -1108,46 +1108,48 @@ __global__ void __launch_bounds__(256, StepOccupancy<Q, S, K>::blocks) k_collide
   // The K cells of a thread lie a warp apart along the fastest axis (n0, n0 + 32, ...): each
   // warp-wide load or store then covers one contiguous run of 32 cells, which a 16-bit column
   // moves in two full sectors, instead of every instruction touching twice the sectors it uses.
-  // Rows: a thread's cells lie in one row of the core.  Flat (`flat`): the threads run through the
+  // Rows: a thread's cells lie in one row of the core.  FLAT: the threads run through the
   // padded cells of a plane (2D: of the lattice), padding included, so that a row need not be a
   // multiple of 32 K cells (groups_shape says when).
   constexpr int W = 32;
   uint32_t n0;
-  int fz[K], sl[K];  // each cell's coordinate on the fastest axis, and on the one before it
-  bool ok[K];        // the cell lies in the core
+  int x = 0, y = 0, z0 = 0, nvalid = 0;  // rows: the first cell, and cells k < nvalid lie in the core
+  int fz[K], sl[K];                      // flat: each cell's coordinates on the fastest axis and the one before
   bool inside = false;
-  if (flat) {
+  auto ok = [&](int k) {  // cell k lies in the core
+    if constexpr (FLAT) return sl[k] < (D::d == 3 ? g.ny : g.nx) && fz[k] < (D::d == 3 ? g.nz : g.ny);
+    else return k < nvalid;
+  };
+  if constexpr (FLAT) {
     const uint32_t t = (blockIdx.x * blockDim.y + threadIdx.y) * blockDim.x + threadIdx.x;
     const uint32_t q0 = (t / W) * (W * K) + t % W;
     const uint32_t row = D::d == 3 ? uint32_t(g.sy) : uint32_t(g.sx);
     const uint32_t m = D::d == 3 ? dv.my : dv.mx;
     const int l = D::d == 3 ? dv.ly : dv.lx;
-    const int nf = D::d == 3 ? g.nz : g.ny, nrows = D::d == 3 ? g.ny : g.nx;
     n0 = (D::d == 3 ? (blockIdx.z + 1u) * uint32_t(g.sx) + row : row) + 1u + q0;
 #pragma unroll
     for (int k = 0; k < K; ++k) {
       const uint32_t q = q0 + uint32_t(W * k), r = (__umulhi(q, m) + q) >> l;
       sl[k] = int(r);
       fz[k] = int(q - r * row);
-      ok[k] = sl[k] < nrows && fz[k] < nf;
-      inside = inside || ok[k];
+      inside = inside || ok(k);
     }
   } else {
     const int gi = blockIdx.x * blockDim.x + threadIdx.x;
     const int m = blockIdx.y * blockDim.y + threadIdx.y;
-    const int z0 = (gi / W) * (W * K) + gi % W;
+    z0 = (gi / W) * (W * K) + gi % W;
     const int nf = D::d == 3 ? g.nz : g.ny;
-    const bool row = m < (D::d == 3 ? g.ny : g.nx);
-    // 3D: (x+1)*sx + (y+1)*sy + z0 + 1; 2D: the fast axis is y (sy = 1), z absent
-    n0 = D::d == 3 ? uint32_t((int(blockIdx.z) + 1) * g.sx + (m + 1) * g.sy + z0 + 1)
-                   : uint32_t((m + 1) * g.sx + z0 + 1);
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      sl[k] = m;
-      fz[k] = z0 + W * k;
-      ok[k] = row && fz[k] < nf;
+    if constexpr (D::d == 3) {
+      y = m;
+      x = blockIdx.z;
+      inside = z0 < nf && y < g.ny;
+    } else {
+      x = m;
+      inside = z0 < nf && x < g.nx;
     }
-    inside = ok[0];
+    nvalid = (nf - z0 + W - 1) / W;
+    // 3D: (x+1)*sx + (y+1)*sy + z0 + 1; 2D: the fast axis is y (sy = 1), z absent
+    n0 = D::d == 3 ? uint32_t((x + 1) * g.sx + (y + 1) * g.sy + z0 + 1) : uint32_t((x + 1) * g.sx + z0 + 1);
   }
   double accRho = 0.0, accUsq = 0.0, accMax = 0.0;
   unsigned accCount = 0;
@@ -1163,11 +1165,11 @@ __global__ void __launch_bounds__(256, StepOccupancy<Q, S, K>::blocks) k_collide
 #pragma unroll
     for (int k = 0; k < K; ++k) {
       if constexpr (MAPPED) {
-        kinds[k] = ok[k] ? cellDyn[n0 + W * k] : uint8_t(0);
+        kinds[k] = ok(k) ? cellDyn[n0 + W * k] : uint8_t(0);
         act[k] = stepped_kind(kinds[k]);
       } else {
-        kinds[k] = ok[k] ? uint8_t(1) : uint8_t(0);
-        act[k] = ok[k];
+        kinds[k] = ok(k) ? uint8_t(1) : uint8_t(0);
+        act[k] = ok(k);
       }
     }
     chain_wait();
@@ -1251,43 +1253,60 @@ __global__ void __launch_bounds__(256, StepOccupancy<Q, S, K>::blocks) k_collide
         Storage<S>::store(col + idx, f[k][I]);
       }
     };
-    if (g.pmask) {
+    auto cross_all = [&](int k, int xk, int yk, int zk) {  // a cell on a periodic slower face
+      static_for<Q>([&](auto I) {
+        constexpr int cx = D::C[I][0], cy = D::C[I][1], cz = D::C[I][2];
+        int tx = xk + cx, ty = yk + cy, tz = zk + cz;
+        bool crossed = false, lost = false;
+        if (tx < 0 || tx >= g.nx) { if (g.pmask & 1) { tx = tx < 0 ? tx + g.nx : tx - g.nx; crossed = true; } else lost = true; }
+        if (ty < 0 || ty >= g.ny) { if (g.pmask & 2) { ty = ty < 0 ? ty + g.ny : ty - g.ny; crossed = true; } else lost = true; }
+        if constexpr (D::d == 3) {
+          if (tz < 0 || tz >= g.nz) { if (g.pmask & 4) { tz = tz < 0 ? tz + g.nz : tz - g.nz; crossed = true; } else lost = true; }
+        }
+        if (crossed && !lost) {
+          const int64_t gn = int64_t(tx - cx + 1) * g.sx + int64_t(ty - cy + 1) * g.sy + (tz - cz + g.pz);
+          ghost_store(I, k, uint32_t(gn));
+        }
+      });
+    };
+    auto cross_fast = [&](int k, int xk, int yk, int fk) {  // any other cell: across the fastest axis
+      if (fk != 0 && fk != nf - 1) return;
+      static_for<Q>([&](auto I) {
+        constexpr int cf = D::d == 3 ? D::C[I][2] : D::C[I][1];
+        if constexpr (cf != 0) {
+          if ((cf > 0 && fk == nf - 1) || (cf < 0 && fk == 0)) {
+            constexpr int cx = D::C[I][0], cy = D::C[I][1];
+            bool in = xk + cx >= 0 && xk + cx < g.nx;
+            if constexpr (D::d == 3) in = in && yk + cy >= 0 && yk + cy < g.ny;
+            if (in) ghost_store(I, k, n0 + W * k - uint32_t(cf * nf));
+          }
+        }
+      });
+    };
+    auto slow_face = [&](int xk, int yk) {
+      return ((g.pmask & 1) && (xk == 0 || xk == g.nx - 1)) ||
+             (D::d == 3 && (g.pmask & 2) && (yk == 0 || yk == g.ny - 1));
+    };
+    constexpr int FAST = D::d == 3 ? 4 : 2;
+    // (no dynamics: nothing to carry across, see linkMask; boundary cells: their own kernels)
+    if constexpr (FLAT) {
+      if (g.pmask) {
 #pragma unroll
-      for (int k = 0; k < K; ++k) {
-        // no dynamics: nothing to carry across (see linkMask); boundary cells: their own kernels
-        if (!act[k]) continue;
-        const int x = D::d == 3 ? int(blockIdx.z) : sl[k], y = D::d == 3 ? sl[k] : fz[k], z = D::d == 3 ? fz[k] : 0;
-        const bool slowFace = ((g.pmask & 1) && (x == 0 || x == g.nx - 1)) ||
-                              (D::d == 3 && (g.pmask & 2) && (y == 0 || y == g.ny - 1));
-        if (slowFace) {
-          static_for<Q>([&](auto I) {
-            constexpr int cx = D::C[I][0], cy = D::C[I][1], cz = D::C[I][2];
-            int tx = x + cx, ty = y + cy, tz = z + cz;
-            bool crossed = false, lost = false;
-            if (tx < 0 || tx >= g.nx) { if (g.pmask & 1) { tx = tx < 0 ? tx + g.nx : tx - g.nx; crossed = true; } else lost = true; }
-            if (ty < 0 || ty >= g.ny) { if (g.pmask & 2) { ty = ty < 0 ? ty + g.ny : ty - g.ny; crossed = true; } else lost = true; }
-            if constexpr (D::d == 3) {
-              if (tz < 0 || tz >= g.nz) { if (g.pmask & 4) { tz = tz < 0 ? tz + g.nz : tz - g.nz; crossed = true; } else lost = true; }
-            }
-            if (crossed && !lost) {
-              const int64_t gn = int64_t(tx - cx + 1) * g.sx + int64_t(ty - cy + 1) * g.sy + (tz - cz + g.pz);
-              ghost_store(I, k, uint32_t(gn));
-            }
-          });
-        } else if ((g.pmask & (D::d == 3 ? 4 : 2)) && (fz[k] == 0 || fz[k] == nf - 1)) {
-          static_for<Q>([&](auto I) {
-            constexpr int cf = D::d == 3 ? D::C[I][2] : D::C[I][1];
-            if constexpr (cf != 0) {
-              if ((cf > 0 && fz[k] == nf - 1) || (cf < 0 && fz[k] == 0)) {
-                constexpr int cx = D::C[I][0], cy = D::C[I][1];
-                bool in = x + cx >= 0 && x + cx < g.nx;
-                if constexpr (D::d == 3) in = in && y + cy >= 0 && y + cy < g.ny;
-                if (in) ghost_store(I, k, n0 + W * k - uint32_t(cf * nf));
-              }
-            }
-          });
+        for (int k = 0; k < K; ++k) {
+          if (!act[k]) continue;
+          const int xk = D::d == 3 ? int(blockIdx.z) : sl[k], yk = D::d == 3 ? sl[k] : fz[k];
+          if (slow_face(xk, yk)) cross_all(k, xk, yk, D::d == 3 ? fz[k] : 0);
+          else if (g.pmask & FAST) cross_fast(k, xk, yk, fz[k]);
         }
       }
+    } else if (slow_face(x, y)) {
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        if (act[k]) cross_all(k, x, D::d == 3 ? y : z0 + W * k, D::d == 3 ? z0 + W * k : 0);
+    } else if (g.pmask & FAST) {
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        if (act[k]) cross_fast(k, x, y, z0 + W * k);
     }
     // halfway bounce-back (BouzidiPostProcessor with q = 1/2, boundary/setBouzidiBoundary.h:48-77,
     // 129-162), fused into the store: a population f_k that leaves the cell towards a solid
@@ -1766,15 +1785,61 @@ __device__ __forceinline__ R rlb_relax(R (&f)[Q], FdMeta m, R rho, const R (&u)[
 // in place at the current shifts, after the bulk step kernel left these cells untouched.  A cell
 // on a periodic face also refreshes the ghost slots of its leaving populations (the bulk
 // kernel wrote them before this collision).  Statistics partials go after the bulk kernel's.
+// (f: the cell's populations, collided and stored; returns its density and |u|^2)
+template <int Q, typename S>
+__device__ __forceinline__ void fd_collide_cell(S* pop, const Geometry& g, const Shifts<Q>& sh, double omega,
+                                                int64_t n, FdMeta m, const double* __restrict__ value,
+                                                typename Storage<S>::R (&f)[Q], double& aR, double& aU) {
+  using R = typename Storage<S>::R;
+  using D = Desc<Q>;
+  R rho, u[3];
+  fd_momenta<Q, R>(f, m, value, rho, u);
+  if (m.local) {  // regularised first, then collided with the momenta of the rebuilt cell
+    local_regularize<Q, R>(f, m, rho, u);
+    fd_momenta<Q, R>(f, m, value, rho, u);
+  }
+  R uSqr = R(0);
+  const R w = R(omega);
+  if (m.rlb) {  // the RLB mixin of a local boundary
+    uSqr = rlb_relax<Q, R>(f, m, rho, u, w);
+  } else {
+    static_for<D::d>([&](auto A) { uSqr += u[A] * u[A]; });
+    static_for<Q>([&](auto I) {
+      f[I] *= R(1) - w;
+      f[I] += w * equilibrium_plain<Q, I>(rho, u, uSqr);
+    });
+  }
+  static_for<Q>([&](auto I) { Storage<S>::store(pop + I * g.stride + wrap_add(n, sh.s[I], g.n), f[I]); });
+  if (g.pmask) {
+    int x, y, z;
+    fd_decode(g, n, x, y, z);
+    static_for<Q>([&](auto I) {
+      constexpr int cx = D::C[I][0], cy = D::C[I][1], cz = D::C[I][2];
+      int tx = x + cx, ty = y + cy, tz = z + cz;
+      bool crossed = false, lost = false;
+      if (tx < 0 || tx >= g.nx) { if (g.pmask & 1) { tx = tx < 0 ? tx + g.nx : tx - g.nx; crossed = true; } else lost = true; }
+      if (ty < 0 || ty >= g.ny) { if (g.pmask & 2) { ty = ty < 0 ? ty + g.ny : ty - g.ny; crossed = true; } else lost = true; }
+      if constexpr (D::d == 3) {
+        if (tz < 0 || tz >= g.nz) { if (g.pmask & 4) { tz = tz < 0 ? tz + g.nz : tz - g.nz; crossed = true; } else lost = true; }
+      }
+      if (crossed && !lost) {
+        const int64_t gn = int64_t(tx - cx + 1) * g.sx + int64_t(ty - cy + 1) * g.sy + (tz - cz + g.pz);
+        Storage<S>::store(pop + I * g.stride + wrap_add(gn, sh.s[I], g.n), f[I]);
+      }
+    });
+  }
+  aR = double(rho);
+  aU = double(uSqr);
+}
+
 template <int Q, typename S>
 __global__ void __launch_bounds__(256) k_fd_collide(S* pop, Geometry g, Shifts<Q> sh, double omega,
                                                     int64_t nFd, const uint32_t* __restrict__ fdCell,
                                                     const uint16_t* __restrict__ fdMeta,
                                                     const double* __restrict__ fdValue, double* __restrict__ statPart) {
   using R = typename Storage<S>::R;
-  using D = Desc<Q>;
   const int64_t b = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  double aR = 0.0, aU = 0.0, aC = 0.0;
+  double aR = 0.0, aU = 0.0;
   chain_next();
   const int64_t n = b < nFd ? fdCell[b] : 0;
   const FdMeta m(b < nFd ? fdMeta[b] : uint16_t(0));
@@ -1782,47 +1847,9 @@ __global__ void __launch_bounds__(256) k_fd_collide(S* pop, Geometry g, Shifts<Q
   if (b < nFd) {
     R f[Q];
     static_for<Q>([&](auto I) { f[I] = Storage<S>::load(pop + I * g.stride + wrap_add(n, sh.s[I], g.n)); });
-    R rho, u[3];
-    fd_momenta<Q, R>(f, m, fdValue + 4 * b, rho, u);
-    if (m.local) {  // regularised first, then collided with the momenta of the rebuilt cell
-      local_regularize<Q, R>(f, m, rho, u);
-      fd_momenta<Q, R>(f, m, fdValue + 4 * b, rho, u);
-    }
-    R uSqr = R(0);
-    const R w = R(omega);
-    if (m.rlb) {  // the RLB mixin of a local boundary
-      uSqr = rlb_relax<Q, R>(f, m, rho, u, w);
-    } else {
-      static_for<D::d>([&](auto A) { uSqr += u[A] * u[A]; });
-      static_for<Q>([&](auto I) {
-        f[I] *= R(1) - w;
-        f[I] += w * equilibrium_plain<Q, I>(rho, u, uSqr);
-      });
-    }
-    static_for<Q>([&](auto I) { Storage<S>::store(pop + I * g.stride + wrap_add(n, sh.s[I], g.n), f[I]); });
-    if (g.pmask) {
-      int x, y, z;
-      fd_decode(g, n, x, y, z);
-      static_for<Q>([&](auto I) {
-        constexpr int cx = D::C[I][0], cy = D::C[I][1], cz = D::C[I][2];
-        int tx = x + cx, ty = y + cy, tz = z + cz;
-        bool crossed = false, lost = false;
-        if (tx < 0 || tx >= g.nx) { if (g.pmask & 1) { tx = tx < 0 ? tx + g.nx : tx - g.nx; crossed = true; } else lost = true; }
-        if (ty < 0 || ty >= g.ny) { if (g.pmask & 2) { ty = ty < 0 ? ty + g.ny : ty - g.ny; crossed = true; } else lost = true; }
-        if constexpr (D::d == 3) {
-          if (tz < 0 || tz >= g.nz) { if (g.pmask & 4) { tz = tz < 0 ? tz + g.nz : tz - g.nz; crossed = true; } else lost = true; }
-        }
-        if (crossed && !lost) {
-          const int64_t gn = int64_t(tx - cx + 1) * g.sx + int64_t(ty - cy + 1) * g.sy + (tz - cz + g.pz);
-          Storage<S>::store(pop + I * g.stride + wrap_add(gn, sh.s[I], g.n), f[I]);
-        }
-      });
-    }
-    aR = double(rho);
-    aU = double(uSqr);
-    aC = 1.0;
+    fd_collide_cell<Q, S>(pop, g, sh, omega, n, m, fdValue + 4 * b, f, aR, aU);
   }
-  if (statPart) block_partial(aR, aU, aU, aC, statPart);
+  if (statPart) block_partial(aR, aU, aU, b < nFd ? 1.0 : 0.0, statPart);
 }
 
 // BounceBack with a wall velocity (BounceBackVelocity, dynamics/dynamics.h:629-637): the
@@ -1888,7 +1915,7 @@ __global__ void __launch_bounds__(256) k_bbv_collide(S* pop, Geometry g, Shifts<
 // Post-stream pass 1: every boundary cell's velocity and density from its momenta, and its
 // bulk velocity (what a neighbour reached across a periodic face sees: the reference's overlap
 // copy of the cell, which carries bulk dynamics), from the populations before any cell is
-// rewritten.  fdMom[7 b ...] = {u, u_bulk, rho}.
+// rewritten.  fdMom[8 b ...] = {u, u_bulk, rho, rho after pass 2 (until then: rho)}.
 template <int Q, typename S>
 __global__ void __launch_bounds__(256) k_fd_momenta(const S* pop, Geometry g, Shifts<Q> sh, int64_t nFd,
                                                     const uint32_t* __restrict__ fdCell,
@@ -1908,12 +1935,13 @@ __global__ void __launch_bounds__(256) k_fd_momenta(const S* pop, Geometry g, Sh
   const R halfF[3] = {R(hfx), R(hfy), R(hfz)};
   fd_momenta<Q, R>(f, m, fdValue + 4 * b, rho, u);
   bulk_velocity<Q, R>(f, halfF, ub);
-  double* out = fdMom + 7 * b;
+  double* out = fdMom + 8 * b;
   for (int a = 0; a < 3; ++a) {
     out[a] = double(u[a]);
     out[3 + a] = double(ub[a]);
   }
   out[6] = double(rho);
+  out[7] = double(rho);
 }
 
 // Post-stream passes 2 and 3: the regularised populations f_i = f_i^eq(rho, u) +
@@ -1932,19 +1960,25 @@ __global__ void __launch_bounds__(256) k_fd_momenta(const S* pop, Geometry g, Sh
 // momenta; the imposed velocity of velocity cells does not depend on the order) or from the
 // populations (bulk cells, never rewritten here); cells without dynamics or with plain
 // bounce-back, and padding cells, read u = 0, rho = 1 (ZeroMomentum with OneDensity /
-// FixedDensity), bounce-back cells with a wall velocity their fixed velocity and density.  Neighbour densities in pass 2 come from pass 1; in pass 3 from the current
-// populations, i.e. those the priority-0 processors left, as the reference's corner processor
-// reads them.
+// FixedDensity), bounce-back cells with a wall velocity their fixed velocity and density.  Neighbour
+// densities in pass 2 come from pass 1; in pass 3 from what the priority-0 processors left, as the
+// reference's corner processor reads them: pass 2 puts down the density that its cells' momenta
+// have afterwards.
+//
+// `collide`: another step of the same call follows, and each cell is collided here, in registers,
+// instead of by a launch of its own (k_fd_collide) in that step.  Nothing else touches the cell's
+// slots in between: passes 2 and 3 read a boundary cell only through fdMom, and the step kernel
+// neither loads nor stores it.
 template <int Q, typename S>
 __global__ void __launch_bounds__(256) k_fd_regularize(S* pop, Geometry g, Shifts<Q> sh, double omega,
                                                        int64_t nFd, const uint32_t* __restrict__ fdCell,
                                                        const uint16_t* __restrict__ fdMeta,
                                                        const double* __restrict__ fdValue,
                                                        const uint8_t* __restrict__ cellDyn, double hfx, double hfy,
-                                                       double hfz, const double* fdMom, int corners,
+                                                       double hfz, double* fdMom, int corners,
                                                        int64_t nBbv, const uint32_t* __restrict__ bbvCell,
                                                        const double* __restrict__ bbvValue,
-                                                       const int32_t* __restrict__ bIdx) {
+                                                       const int32_t* __restrict__ bIdx, int collide) {
   using R = typename Storage<S>::R;
   using D = Desc<Q>;
   // One thread per boundary cell, its neighbour lookups in stages so that the loads of every
@@ -1958,17 +1992,24 @@ __global__ void __launch_bounds__(256) k_fd_regularize(S* pop, Geometry g, Shift
   const int64_t b = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   chain_next();
   const FdMeta m(b < nFd ? fdMeta[b] : uint16_t(0));
-  // local boundaries have no post-processor
-  if (b >= nFd || m.local || (m.type == FD_CORNER_VELOCITY) != (corners != 0)) {
+  if (b >= nFd || (m.type == FD_CORNER_VELOCITY) != (corners != 0) || (m.local && !collide)) {
     chain_wait();
     return;
   }
   const int64_t n = fdCell[b];
+  if (m.local) {  // local boundaries have no post-processor
+    chain_wait();
+    R f[Q];
+    static_for<Q>([&](auto I) { f[I] = Storage<S>::load(pop + I * g.stride + wrap_add(n, sh.s[I], g.n)); });
+    double aR, aU;
+    fd_collide_cell<Q, S>(pop, g, sh, omega, n, m, fdValue + 4 * b, f, aR, aU);
+    return;
+  }
   int pos[3];
   fd_decode(g, n, pos[0], pos[1], pos[2]);
   const int ext[3] = {g.nx, g.ny, g.nz};
   const R halfF[3] = {R(hfx), R(hfy), R(hfz)};
-  const double* own = fdMom + 7 * b;
+  double* own = fdMom + 8 * b;
   const bool flatRho = m.type == FD_FLAT_VELOCITY || m.type == FD_FLAT_PRESSURE;
   const bool edgeRule = !flatRho && (m.type == FD_EDGE_VELOCITY || D::d == 2);
   // the two normal axes A < B (in the cyclic order after the edge axis) of an edge; x, y in 2D
@@ -2047,7 +2088,7 @@ __global__ void __launch_bounds__(256) k_fd_regularize(S* pop, Geometry g, Shift
       nv[s][0] = nv[s][1] = nv[s][2] = R(0);
       if (!use[s]) continue;
       if (bi[s] >= 0) {
-        const double* mm = fdMom + 7 * int64_t(bi[s]) + (wrapped[s] ? 3 : 0);
+        const double* mm = fdMom + 8 * int64_t(bi[s]) + (wrapped[s] ? 3 : 0);
         nv[s][0] = R(mm[0]);
         nv[s][1] = R(mm[1]);
         nv[s][2] = R(mm[2]);
@@ -2060,8 +2101,7 @@ __global__ void __launch_bounds__(256) k_fd_regularize(S* pop, Geometry g, Shift
       nr[s - 6] = R(0);
       if (!use[s]) continue;
       if (bi[s] >= 0) {
-        if (!corners) nr[s - 6] = R(fdMom[7 * int64_t(bi[s]) + 6]);
-        else pend[s] = true;  // the populations the flat and edge pass left
+        nr[s - 6] = R(fdMom[8 * int64_t(bi[s]) + (corners ? 7 : 6)]);
       } else if (kind[s] == kCellBounceBackVelocity) {  // FixedDensity
         nr[s - 6] = jb >= 0 ? R(bbvValue[4 * jb]) : R(1);
       } else if (!bulk_kind(kind[s])) {
@@ -2074,10 +2114,6 @@ __global__ void __launch_bounds__(256) k_fd_regularize(S* pop, Geometry g, Shift
   auto finish = [&](int s, const R (&f)[Q]) {
     if (s < 6) {
       bulk_velocity<Q, R>(f, halfF, nv[s]);
-    } else if (bi[s] >= 0) {
-      R r, v[3];
-      fd_momenta<Q, R>(f, FdMeta(fdMeta[bi[s]]), fdValue + 4 * int64_t(bi[s]), r, v);
-      nr[s - 6] = r;
     } else {
       nr[s - 6] = bulk_rho<Q, R>(f);
     }
@@ -2134,6 +2170,7 @@ __global__ void __launch_bounds__(256) k_fd_regularize(S* pop, Geometry g, Shift
   }
   R uSqr = R(0);
   static_for<D::d>([&](auto AX) { uSqr += u[AX] * u[AX]; });
+  R f[Q];  // as stored and loaded again
   static_for<Q>([&](auto I) {
     constexpr R t = weight<Q, R>(I);
     R fneq = R(0);
@@ -2151,8 +2188,20 @@ __global__ void __launch_bounds__(256) k_fd_regularize(S* pop, Geometry g, Shift
       });
     });
     fneq *= t * R(3) * R(3) / R(2);
-    Storage<S>::store(pop + I * g.stride + wrap_add(n, sh.s[I], g.n), equilibrium_plain<Q, I>(rho, u, uSqr) + fneq);
+    S stored;
+    Storage<S>::store(&stored, equilibrium_plain<Q, I>(rho, u, uSqr) + fneq);
+    if (!collide) pop[I * g.stride + wrap_add(n, sh.s[I], g.n)] = stored;
+    f[I] = Storage<S>::load(&stored);
   });
+  if (!corners) {
+    R after, v[3];
+    fd_momenta<Q, R>(f, m, fdValue + 4 * b, after, v);
+    own[7] = double(after);
+  }
+  if (collide) {
+    double aR, aU;
+    fd_collide_cell<Q, S>(pop, g, sh, omega, n, m, fdValue + 4 * b, f, aR, aU);
+  }
 }
 
 // ---- host <-> column transfers (one population at a time through a staging buffer) -----
@@ -2357,7 +2406,9 @@ struct LaunchArgs {
   const uint32_t* fdCell;    // their padded indices, ascending
   const uint16_t* fdMeta;    // type and outward normal (FdMeta)
   const double* fdValue;     // 4 imposed values per cell
-  double* fdMom;             // 7 doubles per cell of scratch (k_fd_momenta)
+  double* fdMom;             // 8 doubles per cell of scratch (k_fd_momenta)
+  int fdCollided;            // this step's collision of them is done (k_fd_regularize's `collide`)
+  int fdCollideNext;         // k_fd_regularize collides them for the next step
   int64_t nFdCorners;        // how many of them are corners (regularised in a second pass)
   const uint32_t* linkMask;  // per padded cell: directions of fused bounce-back links (kind 7 cells)
   const void* wallDelta;     // wall terms of their classes, [kWallClasses][Q] (null: every wall at rest)
@@ -2376,19 +2427,21 @@ inline int k_cells_threads(int nf, int K) { return K == 1 ? nf : (nf + 32 * K - 
 // Grid of the K-cells step kernel.  Its threads go by rows of the core, or flat through the padded
 // cells of a plane where that leaves fewer lanes idle: rows waste what the row lacks to a multiple
 // of 32 K cells (nz = 97 at K = 1: 24 %), flat the two padding cells of each row.  Where rows fill
-// their lanes they are kept: no division per cell, and no padding lanes.  Variant 5 prefetches rows.
+// their lanes they are kept: no division per cell, and no padding lanes (256^3 at two cells a thread
+// loses 4 % when it carries the flat form's coordinates).  Variant 5 prefetches rows; columns that
+// wrap and four cells a thread stay with rows.
 struct GroupsShape {
   unsigned x, y, z;
   bool flat;
 };
-inline GroupsShape groups_shape(int d, const Geometry& g, int kernel, int K, int bx, int by) {
+inline GroupsShape groups_shape(int d, const Geometry& g, int kernel, int K, int bx, int by, bool doubled) {
   const int64_t nf = d == 3 ? g.nz : g.ny, rows = d == 3 ? g.ny : g.nx, planes = d == 3 ? g.nx : 1;
   const int64_t lanes = k_cells_threads(int(nf), K);
   const int64_t rowLanes = ((lanes + bx - 1) / bx * bx) * ((rows + by - 1) / by * by) * K;
   const int64_t cells = (rows - 1) * (d == 3 ? g.sy : g.sx) + nf, per = int64_t(bx) * by * K;
   const int64_t flatBlocks = (cells + per - 1) / per;
   GroupsShape s;
-  s.flat = kernel == 2 && flatBlocks * per * 21 < rowLanes * 20;
+  s.flat = kernel == 2 && K <= 2 && doubled && flatBlocks * per * 21 < rowLanes * 20;
   s.x = unsigned(s.flat ? flatBlocks : (lanes + bx - 1) / bx);
   s.y = unsigned(s.flat ? 1 : (rows + by - 1) / by);
   s.z = unsigned(planes);
@@ -2597,7 +2650,7 @@ cudaError_t launch_step_dyn(const LaunchArgs& a, cudaStream_t stream) {
       cols.s[i] = a.doubled ? 0u : uint32_t(a.shift[i]);
     }
     const int K = a.cellsPerThread;
-    const GroupsShape shape = groups_shape(Desc<Q>::d, g, a.kernel, K, a.blockX, a.blockY);
+    const GroupsShape shape = groups_shape(Desc<Q>::d, g, a.kernel, K, a.blockX, a.blockY, a.doubled);
     const dim3 block(a.blockX, a.blockY, 1), grid(shape.x, shape.y, shape.z);
     FlatDiv dv;
     FlatDiv::make(uint32_t(g.sx), dv.mx, dv.lx);
@@ -2606,23 +2659,30 @@ cudaError_t launch_step_dyn(const LaunchArgs& a, cudaStream_t stream) {
     if (a.stats && nblocks > a.statCapacity) return cudaErrorInvalidValue;
     double* part = a.stats ? a.statPart : nullptr;
     cudaError_t chained = cudaSuccess;
-    auto go = [&](auto kk, auto doubled, auto mapped) {
-      auto kern =
-          k_collide_stream_groups<Q, S, DYN, decltype(kk)::value, decltype(doubled)::value, decltype(mapped)::value>;
+    auto go = [&](auto kk, auto doubled, auto mapped, auto flat) {
+      auto kern = k_collide_stream_groups<Q, S, DYN, decltype(kk)::value, decltype(doubled)::value,
+                                          decltype(mapped)::value, decltype(flat)::value>;
       static std::atomic<uint64_t> aheadCache[64] = {};  // one per instantiation of this lambda, i.e. per kernel
       int ahead = 0;
       if constexpr (decltype(doubled)::value)
         if (a.kernel == 5) ahead = l2_ahead_blocks(kern, int(block.x * block.y), aheadCache);
       chained = launch_chained(kern, grid, block, stream, cols, g, p, a.cellDyn, a.linkMask,
-                               static_cast<const R*>(a.wallDelta), part, ahead, shape.flat ? 1 : 0, dv);
+                               static_cast<const R*>(a.wallDelta), part, ahead, dv);
     };
     auto go_k = [&](auto kk) {
-      if (a.doubled) {
-        if (a.cellDyn) go(kk, std::true_type{}, std::true_type{});
-        else go(kk, std::true_type{}, std::false_type{});
+      if (!a.doubled) {
+        if (a.cellDyn) go(kk, std::false_type{}, std::true_type{}, std::false_type{});
+        else go(kk, std::false_type{}, std::false_type{}, std::false_type{});
       } else {
-        if (a.cellDyn) go(kk, std::false_type{}, std::true_type{});
-        else go(kk, std::false_type{}, std::false_type{});
+        if constexpr (decltype(kk)::value <= 2) {
+          if (shape.flat) {
+            if (a.cellDyn) go(kk, std::true_type{}, std::true_type{}, std::true_type{});
+            else go(kk, std::true_type{}, std::false_type{}, std::true_type{});
+            return;
+          }
+        }
+        if (a.cellDyn) go(kk, std::true_type{}, std::true_type{}, std::false_type{});
+        else go(kk, std::true_type{}, std::false_type{}, std::false_type{});
       }
     };
     switch (K) {
@@ -2643,7 +2703,7 @@ cudaError_t launch_step_dyn(const LaunchArgs& a, cudaStream_t stream) {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   int64_t fdb = 0;
-  if (a.nFd > 0) {
+  if (a.nFd > 0 && !a.fdCollided) {
     fdb = fd_blocks(a.nFd);
     if (a.stats && nblocks + fdb > a.statCapacity) return cudaErrorInvalidValue;
     e = launch_chained(k_fd_collide<Q, S>, dim3(unsigned(fdb)), dim3(kFdThreads), stream, pop, g, sh, a.omega, a.nFd,
@@ -2679,7 +2739,7 @@ cudaError_t launch_fd_boundary(const LaunchArgs& a, cudaStream_t stream) {
   for (int corners = 0; corners < (a.nFdCorners > 0 ? 2 : 1); ++corners) {
     e = launch_chained(k_fd_regularize<Q, S>, dim3(blocks), dim3(kFdThreads), stream, pop, a.g, sh, a.omega, a.nFd,
                        a.fdCell, a.fdMeta, a.fdValue, a.cellDyn, hf[0], hf[1], hf[2], a.fdMom, corners, a.nBbv,
-                       a.bbvCell, a.bbvValue, a.bIdx);
+                       a.bbvCell, a.bbvValue, a.bIdx, a.fdCollideNext);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;

@@ -32,6 +32,7 @@ def lattice(q, core, periodic, storage, dynamics, solid=0.0, bounce=0.0, lid=Non
         fluid = np.where(ids == lbx.CELL_BULK, 1, np.where(mat == 1, 4, mat)).astype(np.int32)
         lat.set_bouzidi_boundary(fluid, 1, (2, 3), wall_velocity=[(0, 0, 0), lid] if lid is not None else None)
     lat.set_populations((rng.random((q, lat.n_core)) - 0.5) * 1e-2)
+    lat.bulk = (ids == lbx.CELL_BULK).reshape(-1)
     return lat
 
 
@@ -52,12 +53,12 @@ def test_packed_pairs_match_single_cells(dynamics, q, core, storage):
             lat.set_launch_config(variant, 32, 4, cells)
             for _ in range(6):
                 lat.collide_and_stream(1)
-            f = populations(lat)
+            # cells without dynamics hold what streams into them, and a bounce-back cell beside one
+            # returns it to them; variant 1 carries that across a periodic face, variant 2 does not
+            f = populations(lat)[:, lat.bulk]
             assert np.isfinite(f).all()
-            if ref is None:
-                ref = f
-            else:
-                assert np.array_equal(ref, f)
+            ref = f if ref is None else ref
+            assert np.array_equal(ref, f)
 
 
 @pytest.mark.parametrize("storage", ["f64", "f32"])
@@ -109,3 +110,28 @@ def test_fused_moving_walls_match_the_link_kernel(q, core, storage):
         f = populations(lat)
         ref = f if ref is None else ref
         assert np.array_equal(ref, f)
+
+
+@pytest.mark.parametrize("variant", [(2, 64, 2, 1), (1, 64, 2, 1), (0, 256, 1, 1), (3, 256, 1, 1)])
+@pytest.mark.parametrize("storage", ["f64", "f16dev"])
+@pytest.mark.parametrize("name", ["geo_cavity2d_d2q9_ivel_bgk_rest_f64", "geo_cavity_d3q27_ivel_trt_f64",
+                                  "geo_step_d3q19_lvel_bgk_f64", "geo_channel_d3q19_lvel_lpres_f64",
+                                  "geo_channel_d3q27_trt_f64"])
+def test_steps_at_once_match_single_steps_with_boundary_cells(name, storage, variant):
+    """Within a call a step collides the boundary cells for the next one as it rebuilds them; steps
+    called one by one collide them on their own.  The last step's statistics count them either way."""
+    import lbcases as L
+    from test_boundaries import build_from_materials
+    fx = L.load_fixture(name)
+    out = []
+    for chunks in ((1,) * 7, (7,), (3, 4)):
+        lat = build_from_materials(fx, storage)
+        lat.set_launch_config(*variant)
+        lat.set_populations(np.asarray(fx["f0"], np.float64))
+        for i, k in enumerate(chunks):
+            lat.collide_and_stream(k, statistics=i == len(chunks) - 1)
+        stats = lat.get_statistics()
+        out.append((populations(lat), stats))
+    for f, stats in out[1:]:
+        assert np.array_equal(out[0][0], f)
+        assert stats == out[0][1]
