@@ -1043,11 +1043,13 @@ __device__ __forceinline__ R bounced(R f, const R* __restrict__ wall, int i) {
 // warp-wide load reads 64 bytes of a column, and the hint lets L2 fetch the following warps'
 // bytes of the same column with the same DRAM access.  (The line stays in L1: the second cell of
 // a thread, 32 cells on, reads the other half of it; loads that skip L1 ran 23 % slower.)  Wider
-// forms load plainly.
+// forms load plainly.  The statement is volatile and clobbers memory: what it reads is written by
+// the kernel before, so it must stay behind chain_wait() and ahead of the thread's own stores, and
+// without either the compiler may take it for a function of the address alone and move it.
 template <typename S> __device__ __forceinline__ S ld_column(const S* p) {
   if constexpr (sizeof(S) == 2) {
     unsigned short v;
-    asm("ld.global.L2::256B.b16 %0, [%1];" : "=h"(v) : "l"(p));
+    asm volatile("ld.global.L2::256B.b16 %0, [%1];" : "=h"(v) : "l"(p) : "memory");
     S r;
     memcpy(&r, &v, sizeof(v));
     return r;
