@@ -58,7 +58,8 @@ template <> struct Storage<__nv_bfloat16> {
 // such kernel waits in every thread, so a kernel's completion implies that of all before it.  What
 // is set up before the steps (cell kinds, link masks, boundary lists) may be read ahead of the wait;
 // what a kernel of the chain writes is not passed as a __restrict__ pointer, whose loads the compiler
-// may move across the wait.
+// may move across the wait.  A refused launch (a grid the device cannot take) is reported by its own
+// call alone: its error does not stay behind for the check after a later launch.
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -73,7 +74,9 @@ cudaError_t launch_chained(void (*kern)(P...), dim3 grid, dim3 block, cudaStream
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
 }
 
 // ---- geometry of one lattice as the kernels see it -------------------------------------

@@ -113,3 +113,26 @@ def test_cancelling_a_running_request_leaves_the_others_unchanged():
         ra, ua = a.moments(a1)
         rb, ub = b.moments(b1)
         assert np.array_equal(ra, rb) and np.array_equal(ua, ub)
+
+
+def test_a_refused_launch_leaves_no_error_behind():
+    """A launch shape that the device's grid cannot take (more than 65535 blocks of one row along y)
+    fails its own call, before any cell is stepped; the steps after it, of any variant, are those of
+    a lattice that never saw it."""
+    core = (1, 65540, 32)
+    f0 = (np.random.default_rng(5).random((19, int(np.prod(core)))) - 0.5) * 1e-2
+    out = []
+    for refused in (False, True):
+        lat = lbx.BlockLattice(19, core, (1, 1, 1), "f32")
+        lat.define_dynamics("bgk", omega=1.3)
+        lat.set_populations(f0)
+        for variant, block in ((2, (32, 8)), (1, (32, 8)), (5, (32, 8))):
+            if refused:
+                lat.set_launch_config(5, 256, 1, 1)
+                with pytest.raises(lbx.LbxError):
+                    lat.collide_and_stream(1)
+            lat.set_launch_config(variant, *block, 1)
+            lat.collide_and_stream(2)
+        out.append(lat.get_populations())
+        lat.close()
+    assert np.array_equal(out[0], out[1])
