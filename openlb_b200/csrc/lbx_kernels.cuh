@@ -292,8 +292,14 @@ __device__ __forceinline__ CollisionParams<R> class_params(const ClassParams<R>&
   return r;
 }
 
+// Resident blocks variant 1 is compiled for (0: the compiler's choice).  The call of collide_kind
+// brings the registers of its widest collision into every kernel: 48 on D2Q9 with FP32 arithmetic,
+// whose own collision needs 40 (2048^2 with classes: 99 us a step with 48, 86 with 40).
+template <int Q, typename S> struct StepOccupancy1 {
+  static constexpr int blocks = Q == 9 && sizeof(typename Storage<S>::R) == 4 ? 6 : 0;
+};
 template <int Q, typename S, int DYN>
-__global__ void __launch_bounds__(256) k_collide_stream(S* __restrict__ pop, Geometry g, Shifts<Q> sh,
+__global__ void __launch_bounds__(256, StepOccupancy1<Q, S>::blocks) k_collide_stream(S* __restrict__ pop, Geometry g, Shifts<Q> sh,
                                                         CollisionParams<typename Storage<S>::R> p,
                                                         const uint8_t* __restrict__ cellDyn,
                                                         double* __restrict__ statPart,
@@ -326,10 +332,12 @@ __global__ void __launch_bounds__(256) k_collide_stream(S* __restrict__ pop, Geo
     if (bulk_kind(kind)) {
       if (cls.used && kind >= kCellClassFirst) {
         const int c = int(kind) - kCellClassFirst;
-        const CollisionParams<R> pc = class_params(cls, c);
         const int cd = c == 0 ? cls.dyn[0] : (c == 1 ? cls.dyn[1] : cls.dyn[2]);
-        if (cd == 0 || cd == DYN) collide<Q, R, DYN>(f, pc, rho, usq);
-        else collide_kind<Q, R>(cd, f, pc, rho, usq);
+        // each branch selects for itself: a set of parameters shared by both goes through local
+        // memory, for the call's sake, in the inlined collision as well (FP64 D3Q19 192^3: 623 us a
+        // step so, 571 with two selections)
+        if (cd == 0 || cd == DYN) collide<Q, R, DYN>(f, class_params(cls, c), rho, usq);
+        else collide_kind<Q, R>(cd, f, class_params(cls, c), rho, usq);
       } else {
         collide<Q, R, DYN>(f, p, rho, usq);
       }
