@@ -1001,7 +1001,7 @@ int step_post_stream(lbx_lattice_s* L, cudaStream_t s, bool fdCollideNext = fals
   if (L->nLinks > 0 || L->nFd > 0) {
     LaunchArgs b = args_of(L);
     b.fdCollideNext = fdCollideNext ? 1 : 0;
-    // the K-cells kernel applied the resting links itself (linkMask); the link kernel does
+    // the K-cells kernel applied the fused links itself (linkMask); the link kernel does
     // the rest, or all of them after the other kernel variants
     if (b.linkMask) {
       if (L->nRest > 0)

@@ -761,7 +761,7 @@ __global__ void __launch_bounds__(BulkCfg<Q, S>::THREADS, BulkCfg<Q, S>::BLOCKS)
 //     stores have read it (the store group one behind the newest), so NS - 1 tiles are in flight
 //     ahead of the one being computed;
 //   - warps 1..16 are consumers: each waits for its tile's `full` phase, collides its cells in
-//     shared memory (16-bit BGK pairs with the packed two-cell collision), writes the unaligned
+//     shared memory (16-bit pairs with the packed two-cell collision, all but ConstRhoBGK's), writes the unaligned
 //     head and tail elements of each run straight to their slots, makes its shared-memory
 //     writes visible to the bulk-copy proxy and arrives on the stage's `empty` barrier.
 // A fast consumer warp runs ahead into the next loaded stage instead of waiting for the block.
@@ -1003,8 +1003,9 @@ __global__ void __launch_bounds__(WsCfg<Q, S>::THREADS, WsCfg<Q, S>::BLOCKS) k_c
 // 2D).  For every population it forms ONE wrapped column index; the K values are then reached
 // with constant offsets (a separate per-element wrap is only needed in the rare group that
 // straddles the cyclic end of the column).  All K*Q loads are issued before the first
-// collision.  Periodic faces are handled by k_periodic_halo after this kernel, so the hot
-// kernel carries no face logic.  Column indices are 32-bit: the column period is < 2^31.
+// collision.  Cells on periodic faces write the ghost slots of what leaves them here, so that a
+// step needs no k_periodic_halo after this kernel.  Column indices are 32-bit: the column period is
+// < 2^31.
 template <int Q>
 struct ColumnBases {
   void* base[Q];   // start of population column i (doubled columns: start + shift)
@@ -1013,15 +1014,15 @@ struct ColumnBases {
 
 // Resident blocks per SM the step kernel is compiled for: the 16-bit forms move half the
 // bytes per request, so they need more warps in flight to keep HBM busy.  D3Q27 at one cell
-// per thread (16-bit and FP32): four blocks (64 registers, no spills; for the 16-bit forms
-// 24-38 % faster than the compiler's 96-142 registers for TRT and Smagorinsky-forced BGK); at
-// six blocks its 27 values spill.
+// per thread (16-bit and FP32): four blocks (64 registers; without a cell map all but 8 bytes stay
+// in them, with one 64-176 bytes spill; for the 16-bit forms 24-38 % faster than the compiler's
+// 96-142 registers for TRT and Smagorinsky-forced BGK); at six blocks its 27 values spill.
 template <int Q, typename S, int K> struct StepOccupancy { static constexpr int blocks = 1; };
 template <> struct StepOccupancy<19, __half, 1> { static constexpr int blocks = 4; };
 template <> struct StepOccupancy<19, __nv_bfloat16, 1> { static constexpr int blocks = 4; };
 template <> struct StepOccupancy<27, float, 1> { static constexpr int blocks = 4; };
 // FP64 D3Q19, one cell per thread: three blocks (80 registers) run 2-3 % faster than the
-// compiler's choice (FP32 at two cells per thread is fastest with its own 96 registers)
+// compiler's choice (FP32 at two cells per thread is left with its own 104-112)
 template <> struct StepOccupancy<19, double, 1> { static constexpr int blocks = 3; };
 template <> struct StepOccupancy<27, __half, 1> { static constexpr int blocks = 4; };
 template <> struct StepOccupancy<27, __nv_bfloat16, 1> { static constexpr int blocks = 4; };
@@ -1802,9 +1803,13 @@ __device__ __forceinline__ R rlb_relax(R (&f)[Q], FdMeta m, R rho, const R (&u)[
 
 // Collision of the boundary cells: BGKdynamics with the boundary momenta
 // (collision::BGK::apply with lbm::bgkCollision, dynamics/collision.h:68-78, lbm.h:395-403),
-// in place at the current shifts, after the bulk step kernel left these cells untouched.  A cell
-// on a periodic face also refreshes the ghost slots of its leaving populations (the bulk
-// kernel wrote them before this collision).  Statistics partials go after the bulk kernel's.
+// in place at the current shifts.  Called by k_fd_collide, after the step kernel, and by
+// k_fd_regularize with `collide`, at the end of the step before and so ahead of the step kernel.
+// Either order gives the same populations: the K-cells kernel neither loads nor stores these cells,
+// the other variants put back what they loaded.  A cell on a periodic face also writes the ghost
+// slots of its leaving populations.  A ghost slot has one source cell, so no store of the step
+// kernel meets them; k_periodic_halo, where a variant needs it, writes the same values once more.
+// Statistics partials (k_fd_collide) go after the bulk kernel's.
 // (f: the cell's populations, collided and stored; returns its density and |u|^2)
 template <int Q, typename S>
 __device__ __forceinline__ void fd_collide_cell(S* pop, const Geometry& g, const Shifts<Q>& sh, double omega,
