@@ -44,11 +44,14 @@ def populations(lat):
 
 @pytest.mark.parametrize("dynamics", DYNAMICS)
 @pytest.mark.parametrize("q,core,storage", [(19, (5, 6, 67), "f32"), (27, (4, 5, 97), "f16dev"),
-                                            (9, (7, 130), "f32"), (19, (3, 4, 33), "bf16dev")])
+                                            (9, (7, 130), "f32"), (19, (3, 4, 33), "bf16dev"),
+                                            (19, (3, 4, 64), "f32"), (9, (8, 128), "f32"), (9, (5, 96), "f16dev")])
 def test_packed_pairs_match_single_cells(dynamics, q, core, storage):
+    """Variant 2 runs rows of a multiple of 64 cells as rows and the ragged ones flat; variant 5 runs
+    them all as rows, with lanes and second cells beyond a row's end."""
     for kw in ({}, {"solid": 0.3}, {"bounce": 0.1, "solid": 0.1}):
         ref = None
-        for variant, cells in ((1, 1), (2, 1), (2, 2)):
+        for variant, cells in ((1, 1), (2, 1), (2, 2), (5, 1), (5, 2)):
             lat = lattice(q, core, (1, 1, 1 if q != 9 else 0), storage, dynamics, **kw)
             lat.set_launch_config(variant, 32, 4, cells)
             for _ in range(6):
@@ -81,15 +84,17 @@ def test_ragged_rows_match_one_thread_per_cell(q, core, storage):
 
 
 @pytest.mark.parametrize("storage", ["f64", "f32", "f16dev"])
-@pytest.mark.parametrize("q,core", [(19, (9, 8, 34)), (27, (6, 7, 33)), (9, (20, 37))])
+@pytest.mark.parametrize("q,core", [(19, (9, 8, 34)), (19, (5, 9, 67)), (19, (5, 8, 64)), (27, (6, 7, 33)), (9, (40, 37)),
+                                    (9, (35, 64))])
 def test_fused_moving_walls_match_the_link_kernel(q, core, storage):
-    """Links of a moving wall, fused into the step's store, against the link kernel (variant 1); with
-    a wall velocity that differs from cell to cell there are more wall terms than classes, and the
-    step fuses some and leaves the others."""
+    """Links of a moving wall, fused into the step's store, against the link kernel (variant 1), with
+    one and two cells a thread, by rows and flat; with a wall velocity that differs from cell to cell
+    there are more wall terms than classes, and the step fuses some and leaves the others."""
+    configs = ((1, 32, 8, 1), (2, 32, 8, 1), (2, 64, 4, 1), (2, 32, 4, 2), (5, 32, 8, 1), (5, 32, 4, 2))
     ref = None
-    for variant, block in ((1, (32, 8)), (2, (32, 8)), (2, (64, 4))):
+    for config in configs:
         lat = lattice(q, core, (0, 0, 0), storage, "bgk", solid=0.1, lid=(0.05, 0.0, 0.01))
-        lat.set_launch_config(variant, *block, 1)
+        lat.set_launch_config(*config)
         lat.post_process()
         for _ in range(5):
             lat.collide_and_stream(1)
@@ -97,14 +102,15 @@ def test_fused_moving_walls_match_the_link_kernel(q, core, storage):
         ref = f if ref is None else ref
         assert np.array_equal(ref, f)
     ref = None
-    for variant in (1, 2):
+    for config in configs:
         lat = lattice(q, core, (0, 0, 0), storage, "bgk", lid=(0.05, 0.0, 0.01))
         mat = np.ones(lat.core, np.int32)
         mat[:, -1, :] = 3
         cells, dirs, wall = lbx.build_bouzidi_links(q, lat.core, mat, 1, (3,), [(1.0, 0.0, 0.0)])
+        assert len(np.unique(cells[wall != 0])) > 31
         wall = wall * (0.02 + 1e-4 * np.arange(len(cells)))
         lat.set_bouzidi_links(cells, dirs, wall)
-        lat.set_launch_config(variant, 32, 8, 1)
+        lat.set_launch_config(*config)
         for _ in range(5):
             lat.collide_and_stream(1)
         f = populations(lat)
@@ -133,7 +139,8 @@ def test_wall_terms_are_told_apart_bit_for_bit():
         assert np.array_equal(ref, f, equal_nan=True)
 
 
-@pytest.mark.parametrize("variant", [(2, 64, 2, 1), (1, 64, 2, 1), (0, 256, 1, 1), (3, 256, 1, 1)])
+@pytest.mark.parametrize("variant", [(2, 64, 2, 1), (2, 32, 4, 2), (5, 32, 8, 1), (5, 32, 4, 2), (1, 64, 2, 1),
+                                     (0, 256, 1, 1), (3, 256, 1, 1)])
 @pytest.mark.parametrize("storage", ["f64", "f16dev"])
 @pytest.mark.parametrize("name", ["geo_cavity2d_d2q9_ivel_bgk_rest_f64", "geo_cavity_d3q27_ivel_trt_f64",
                                   "geo_step_d3q19_lvel_bgk_f64", "geo_channel_d3q19_lvel_lpres_f64",
