@@ -185,7 +185,6 @@ struct lbx_lattice_s {
   int blockX = 256, blockY = 1;
   int kernel = 2;
   int cellsPerThread = 1;
-  bool shapeChosen = false;  // by the caller, the autotuner or a parameter class; else default_block_shape's
   int64_t bytes = 0;
   // optional per-kernel event timing (lbx_set_kernel_timing)
   bool timing = false;
@@ -311,22 +310,22 @@ void block_shape_for(int nf, int cellsPerThread, int threads, int& bx, int& by) 
   by = threads / bx;
 }
 
-// The shape a lattice steps with until one is chosen (lbx_set_launch_config, lbx_autotune): the K-cells
-// kernel in blocks of 128 threads (at 256^3 and 96^3 as fast as 256 in FP64 and 3-11 % faster in FP32
-// and FP16: the tail of a launch is shorter), with one or two cells a thread.  One cell's time over
-// two cells', in a periodic box and in a lid-driven cavity:
-//   FP16 D3Q19   64^3 0.87, 80^3 1.00, 104^3 1.08 and 1.02, 128^3 1.15 and 1.19, 160^3 1.08 and 1.04,
-//                256^3 1.07 and 1.15; 40 % solid blocks 0.94 at 112^3, 1.00 at 192^3, 1.28 at 256^3
+// The shape a lattice starts with: the K-cells kernel in blocks of 128 threads (at 256^3 and 96^3 as
+// fast as 256 in FP64 and 3-11 % faster in FP32 and FP16: the tail of a launch is shorter), with one
+// or two cells a thread.  One cell's time over two cells', in a periodic box and in a lid-driven
+// cavity, BGK where no other is named:
+//   FP16 D3Q19   64^3 0.87 and 1.00, 80^3 1.00, 104^3 1.08 and 1.02, 128^3 1.15 and 1.19, 160^3 1.08 and
+//                1.04, 256^3 1.07 and 1.18; 40 % solid blocks 0.94 at 112^3, 1.00 at 192^3, 1.28 at 256^3
 //   FP16 D2Q9    1000^2 1.24 and 1.12, 2048^2 1.39 and 1.14, 4096^2 1.24 and 1.04
 //   FP32 D2Q9    1024^2 1.08 and 1.07, 1700^2 0.96 and 0.93, 2048^2 1.10 and 1.01, 3000^2 1.11 and 1.02
-//   FP32 D3Q19   104^3 0.87 and 0.88, 160^3 0.98 and 0.95, 288^3 0.95 and 0.95, TRT 0.78 at 112^3 to 224^3;
-//                128^3 0.99 and 0.95, TRT 1.04 and 0.93; 256^3 1.01 and 0.97, TRT 1.06 and 0.97;
-//                64 x 64 x 256 0.92, TRT 0.94; 192 x 192 x 128 1.01, TRT 1.06
+//   FP32 D3Q19   rows that fill their lanes in pairs: 64 x 64 x 256 0.92, 128^3 1.00 and 1.02, 192 x 192 x
+//                128 1.01 and 1.04, 256^3 1.00 and 1.05, 40 % solid 1.06; TRT 1.04 to 1.07 in boxes; forced
+//                Smagorinsky 1.04 to 1.06 in boxes, 0.94 to 0.98 with a map.  Other rows: 104^3 0.88 and
+//                0.88, 160^3 0.98 and 0.91, 288^3 0.96 and 0.90, TRT 0.78 in every box
 //   FP64 D3Q19   104^3 0.93 and 0.89, 160^3 0.96 and 0.85
 // So two on 2^20 cells and more for the 16-bit forms of D3Q19 and D2Q9 and for FP32 D2Q9, and on 2^21
-// and more for FP32 D3Q19 without a cell map on rows that fill their lanes in pairs (others run flat,
-// where the pairs' registers cost more than they bring).  D3Q27 loses 10-18 % to its registers at any
-// size.
+// and more for FP32 D3Q19 on filled rows (others run flat, where the pairs' registers cost more than
+// they bring).  D3Q27 loses 10-18 % to its registers at any size.
 void default_block_shape(lbx_lattice_s* L) {
   const int nf = (L->d == 3) ? L->core[2] : L->core[1];
   L->kernel = (L->period < (int64_t(1) << 31)) ? 2 : 1;
@@ -334,9 +333,8 @@ void default_block_shape(lbx_lattice_s* L) {
   if (L->kernel == 2 && L->ncore >= (int64_t(1) << 20) && L->q != 27 && L->storage != LBX_F64) {
     int bx, by;
     block_shape_for(nf, 2, 128, bx, by);
-    const bool filled = nf % (2 * bx) == 0, mapped = !L->hostMap.empty() || L->nLinks > 0;
-    if (storage_bytes(L->storage) == 2 || L->q == 9 || (filled && !mapped && L->ncore >= (int64_t(1) << 21)))
-      L->cellsPerThread = 2;
+    const bool filled = nf % (2 * bx) == 0 && L->ncore >= (int64_t(1) << 21);
+    if (storage_bytes(L->storage) == 2 || L->q == 9 || filled) L->cellsPerThread = 2;
   }
   const int64_t rows = (L->d == 3) ? L->core[1] : L->core[0];
   block_shape_for(nf, L->cellsPerThread, L->kernel == 2 ? 128 : 256, L->blockX, L->blockY);
@@ -674,7 +672,6 @@ std::vector<double> wall_classes(const lbx_lattice_s* L, std::vector<uint8_t>& f
 // the other kernel variants applies all links.
 int refresh_cell_map(lbx_lattice_s* L) {
   ++L->mapVersion;
-  if (!L->shapeChosen) default_block_shape(L);  // it goes by whether there is a map
   if (int rc = refresh_boundary_index(L)) return rc;
   const bool need = !L->hostMap.empty() || L->nLinks > 0;
   cudaFree(L->linkMask);
@@ -1182,12 +1179,11 @@ int lbx_set_dynamics_class(lbx_lattice L, int32_t cls, const lbx_params* params)
   L->classDyn[cls - 1] = 0;
   L->classMask |= 1 << (cls - 1);
   // the classes run on the one-cell-per-thread step kernel, in the blocks the lattice has: the
-  // default ones of 128 threads, whole or half a row of it wide, are within 3 % of each other and
-  // as fast as 256 threads or faster (192^3 D3Q19 FP32 324-345 us against 339-358, FP64 624-647
-  // against 652-718; FP16 287-302 against 295-321)
+  // default ones of 128 threads (32, 64 or 128 wide) are as fast as 256 threads or faster (192^3 D3Q19
+  // FP32 305-331 us against 324-343, FP64 557-605 against 607-670, FP16 276-293 against 284-313; 2048^2
+  // FP32 89-93 against 93-94)
   L->kernel = 1;
   L->cellsPerThread = 1;
-  L->shapeChosen = true;
   return LBX_OK;
 }
 
@@ -1792,7 +1788,6 @@ int lbx_set_launch_config(lbx_lattice L, int32_t variant, int32_t block_x, int32
   }
   L->cellsPerThread = groups_kernel(variant) ? cells_per_thread : 1;
   L->kernel = variant;
-  L->shapeChosen = true;
   return LBX_OK;
 }
 
@@ -1832,7 +1827,6 @@ int lbx_autotune(lbx_lattice L, int32_t steps, lbx_tune_entry* out, int32_t capa
   }
   if (n_out) *n_out = int32_t(cands.size());
   const Cand keep{L->kernel, L->blockX, L->blockY, L->cellsPerThread};
-  const bool chosen = L->shapeChosen;
   // saved state: every column's period of populations and the shifts
   const size_t es = storage_bytes(L->storage);
   const size_t colBytes = size_t(L->period) * es, pitch = size_t(L->stride) * es;
@@ -1903,7 +1897,6 @@ int lbx_autotune(lbx_lattice L, int32_t steps, lbx_tune_entry* out, int32_t capa
   L->blockX = pick.bx;
   L->blockY = pick.by;
   L->cellsPerThread = pick.k;
-  if (best < 0) L->shapeChosen = chosen;
   if (rc != LBX_OK) return fail(rc, "autotune: " + err);
   if (e != cudaSuccess) return fail(LBX_ERR_CUDA, std::string("autotune: ") + cudaGetErrorString(e));
   return LBX_OK;
